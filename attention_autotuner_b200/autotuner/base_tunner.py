@@ -287,13 +287,16 @@ class BaseTunner:
         return os.path.join(self.cache_path, "best_config_{}_{}_{}{}.json".format(
             self.op_name, self.problem_key["dim_qk"], self.problem_key["dim_v"], self._key_suffix()))
 
+    def cache_candidates(self) -> list:
+        """Files check_cache reads, in its order."""
+        return [self._cache_file(), os.path.join(self.cache_path, "best_config_{}_{}_{}.json".format(
+            self.op_name, self.problem_key["dim_qk"], self.problem_key["dim_v"]))]
+
     def check_cache(self):
         """Best configuration from cache/best_config_<op>_<dqk>_<dv>_sm<cc>_<dtype>[_causal].json; the
         reference's coarser key (base_tunner.py:192,202: op, dqk, dv only) is read as a fallback when it holds
         a configuration of this package."""
-        old_style = os.path.join(self.cache_path, "best_config_{}_{}_{}.json".format(
-            self.op_name, self.problem_key["dim_qk"], self.problem_key["dim_v"]))
-        for path in (self._cache_file(), old_style):
+        for path in self.cache_candidates():
             try:
                 mtime = os.stat(path).st_mtime_ns
             except OSError:

@@ -75,6 +75,49 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     return LIB_PATH
 
 
+# The native operator layer (csrc/host/torch_ops.cpp): a CPython extension against the installed PyTorch's headers, no
+# CUDA code of its own. It is loaded by ops/_native.py.
+OPS_SRC = os.path.join(CSRC, "host", "torch_ops.cpp")
+OPS_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_torch_ops.so")
+
+
+def _ops_hash() -> str:
+    import hashlib
+    import torch
+    h = hashlib.sha1(f"{torch.__version__} {sys.version_info[:2]}".encode())
+    with open(OPS_SRC, "rb") as f:
+        h.update(f.read())
+    return h.hexdigest()
+
+
+def build_torch_ops(force: bool = False) -> str:
+    """Compiles csrc/host/torch_ops.cpp into _torch_ops.so; rebuilt when the source or the PyTorch version changes."""
+    stamp = OPS_PATH + ".srchash"
+    want = _ops_hash()
+    try:
+        with open(stamp) as f:
+            fresh = f.read().strip() == want
+    except OSError:
+        fresh = False
+    if not force and fresh and os.path.exists(OPS_PATH):
+        return OPS_PATH
+    import sysconfig
+    import torch
+    cuda_home = os.path.dirname(os.path.dirname(os.path.realpath(NVCC)))
+    torch_dir = os.path.dirname(torch.__file__)
+    incs = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+            os.path.join(cuda_home, "include"), sysconfig.get_paths()["include"]]
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{d}" for d in incs], OPS_SRC, "-o", OPS_PATH,
+           f"-L{os.path.join(torch_dir, 'lib')}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
+    with open(stamp, "w") as f:
+        f.write(want + "\n")
+    return OPS_PATH
+
+
 BENCH_DIR = os.path.join(os.path.dirname(os.path.abspath(__file__)), "benchmarks")
 BENCH_PROGRAMS = {"attention_bench": "attention.cu", "retnet_bench": "retnet.cu"}
 
@@ -116,5 +159,6 @@ def build_benchmarks(force: bool = False) -> list:
 
 if __name__ == "__main__":
     print(build_library(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_torch_ops(force="--force" in sys.argv))
     if "--benchmarks" in sys.argv:
         print("\n".join(build_benchmarks(force="--force" in sys.argv)))

@@ -1,0 +1,119 @@
+"""The native operator layer (csrc/host/torch_ops.cpp, built into _torch_ops.so) and the plans it is called with.
+
+A plan names the per-configuration library entry point that serves a call. It is resolved by the tuner exactly as before
+(tuning-cache file, search, or the built-in tile) and remembered per (operation, head dimensions, dtype, mask form)
+together with everything the choice was read from: the cache files' modification times and the environment variables.
+The native layer compares those on every call (two ``stat`` calls) and refuses a stale plan, so a cache entry written
+by this or another process takes effect at the next call, as it did when the tuner ran on every call."""
+from __future__ import annotations
+
+import ctypes
+import importlib.machinery
+import importlib.util
+import os
+import threading
+
+import torch
+
+from .. import _lib
+from ..autotuner.runtime import KernelError, Runtime
+from ..autotuner.tunner import AttnTunner, RetBwdTunner, RetTunner
+from ..build import OPS_PATH
+
+_ENV = ["ATTN_B200_CACHE_DIR", "ATTN_B200_AUTOTUNE"]
+
+_lock = threading.Lock()
+_module = None
+_plans: dict = {}
+_archs: list = []  # device descriptions seen by RetNet calls: the backward resolves its plan with the forward's
+
+
+def _address(fn) -> int:
+    return ctypes.cast(fn, ctypes.c_void_p).value
+
+
+def ops():
+    """The native module; raises if it has not been built (python -m attention_autotuner_b200.build)."""
+    global _module
+    if _module is not None:
+        return _module
+    with _lock:
+        if _module is None:
+            if not os.path.exists(OPS_PATH):
+                raise RuntimeError(f"{OPS_PATH} is missing: build it with `python -m attention_autotuner_b200.build`. "
+                                   "There is no fallback.")
+            loader = importlib.machinery.ExtensionFileLoader("_torch_ops", OPS_PATH)
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_torch_ops", loader))
+            loader.exec_module(mod)
+            lib = _lib.load()
+            mod.init(KernelError, _lib.AttnB200Error, _resolve_bwd, _address(lib.attn_b200_last_error),
+                     _address(lib.attn_b200_fa_bwd), _address(lib.attn_b200_ret_chunk_workspace_bytes),
+                     _address(lib.attn_b200_ret_chunk_fwd_ws))
+            _module = mod
+    return _module
+
+
+def _resolve(tuner, key):
+    """Plan of the configuration the tuner picks. Remembered unless the pick was neither read from the tuning cache nor
+    the built-in tile by request (then the tuner is asked again next time, as a failed search should be)."""
+    cfg = tuner.tune()
+    rt = Runtime(tuner.arch, cfg)
+    lib = rt._lib()
+    plan = ops().make_plan(_address(lib.kernel_entry_ex), _address(lib.last_error), rt.libname, tuner.cache_candidates(), _ENV)
+    if tuner.check_cache() is not None or os.environ.get("ATTN_B200_AUTOTUNE", "1") == "0":
+        _plans[key] = plan
+    return plan
+
+
+def _key(op, arch, dqk, dv, dtype, flag):
+    return (op, type(arch), arch.compute_capability, dqk, dv, dtype, flag)
+
+
+def attn_plan(arch, q, v, causal):
+    return _plans.get(_key("attn", arch, q.shape[-1], v.shape[-1], q.dtype, bool(causal)))
+
+
+def resolve_attn(arch, q, k, v, causal, scale):
+    o = torch.empty(*q.shape[:3], v.shape[3], device=q.device, dtype=q.dtype)  # a search times the kernels on these tensors
+    tuner = AttnTunner(arch=arch, torch_array=[q.detach().contiguous(), k.detach().contiguous(), v.detach().contiguous(), o],
+                       scale=scale, causal=causal)
+    return _resolve(tuner, _key("attn", arch, q.shape[-1], v.shape[-1], q.dtype, bool(causal)))
+
+
+def _ret_flag(causal, has_decay):
+    return "decay" if has_decay else bool(causal)  # what the tuner's cache key depends on
+
+
+def ret_plan(op, arch, q, v, causal, decay):
+    return _plans.get(_key(op, arch, q.shape[-1], v.shape[-1], q.dtype, _ret_flag(causal, decay is not None)))
+
+
+def resolve_ret(arch, q, k, v, mask, causal, scale, decay):
+    q, k, v = (t.detach().contiguous() for t in (q, k, v))
+    mask = mask.detach().contiguous() if mask is not None else None
+    if decay is not None:
+        decay = decay.detach().to(device=q.device, dtype=torch.float32).contiguous().reshape(-1)
+    o = torch.empty(*q.shape[:3], v.shape[3], device=q.device, dtype=q.dtype)
+    r = torch.empty(q.shape[:3], device=q.device, dtype=torch.float32)
+    tuner = RetTunner(arch=arch, torch_array=[q, k, v, mask, o, r], scale=scale, causal=causal, decay=decay)
+    return _resolve(tuner, _key("ret", arch, q.shape[-1], v.shape[-1], q.dtype, _ret_flag(causal, decay is not None)))
+
+
+def arch_token(arch) -> int:
+    """Small integer under which the backward finds the device description of its forward."""
+    for i, a in enumerate(_archs):
+        if a is arch or (type(a) is type(arch) and a.__dict__ == arch.__dict__):
+            return i
+    with _lock:
+        _archs.append(arch)
+        return len(_archs) - 1
+
+
+def _resolve_bwd(token, arr, scale, causal, decay):
+    """Called by the native backward when it has no valid plan: arr = [q, k, v, mask, do, r, dq, dk, dv, scratch]."""
+    arch = _archs[token]
+    key = _key("ret_bwd", arch, arr[0].shape[-1], arr[2].shape[-1], arr[0].dtype, _ret_flag(causal, decay is not None))
+    plan = _plans.get(key)
+    if plan is not None and ops().plan_fresh(plan):
+        return plan
+    return _resolve(RetBwdTunner(arch=arch, torch_array=list(arr), scale=scale, causal=causal, decay=decay), key)

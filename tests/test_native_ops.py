@@ -1,0 +1,75 @@
+"""The native operator layer (csrc/host/torch_ops.cpp): staleness of plans without a GPU; autograd errors and strided
+gradients through the operators on one."""
+import os
+
+import pytest
+import torch
+
+
+def test_plan_goes_stale_with_its_files_and_environment(tmp_path, monkeypatch):
+    from attention_autotuner_b200.ops import _native
+    native = _native.ops()
+    f = tmp_path / "best.json"
+    monkeypatch.delenv("ATTN_B200_X", raising=False)
+    plan = native.make_plan(0, 0, "lib", [str(f), str(tmp_path / "other.json")], ["ATTN_B200_X"])
+    assert native.plan_fresh(plan)
+    monkeypatch.setenv("ATTN_B200_X", "1")
+    assert not native.plan_fresh(plan)
+    monkeypatch.delenv("ATTN_B200_X")
+    assert native.plan_fresh(plan)
+    f.write_text("{}")
+    assert not native.plan_fresh(plan)
+    plan = native.make_plan(0, 0, "lib", [str(f)], [])
+    assert native.plan_fresh(plan)
+    os.utime(f, ns=(1, 1))
+    assert not native.plan_fresh(plan)
+    assert not native.plan_fresh(None)
+
+
+def test_declines_what_the_python_checks_word():
+    from attention_autotuner_b200.arch import B200
+    from attention_autotuner_b200.ops import _native
+    from attention_autotuner_b200.ops.attention_interface import flash_attn_func
+    from attention_autotuner_b200.ops.retnet_interface import RetNetAttnFunc, retnet_chunkwise
+    native = _native.ops()
+    q = torch.zeros(1, 2, 8, 128, dtype=torch.float16)  # not on a CUDA device
+    plan = native.make_plan(0, 0, "lib", [], [])
+    assert native.attn(q, q, q, plan, 1.0, False, False) is None
+    assert native.retnet(q, q, q, None, torch.ones(2), plan, None, 0, 1.0, True) is None
+    assert native.chunkwise(q, q, q, torch.ones(2), 1.0) is None
+    for call in (lambda: flash_attn_func(q, q, q, B200()), lambda: flash_attn_func(None, q, q, B200()),
+                 lambda: RetNetAttnFunc(q, q, q, None, B200(), decay=torch.ones(2)),
+                 lambda: retnet_chunkwise(q, q, q, torch.ones(2))):
+        with pytest.raises(ValueError):
+            call()
+
+
+@pytest.mark.gpu
+def test_backward_errors_keep_their_class_and_strided_gradients_are_taken():
+    from attention_autotuner_b200.arch import B200
+    from attention_autotuner_b200.ops.attention_interface import flash_attn_func
+    from attention_autotuner_b200.ops.retnet_interface import RetNetAttnFunc
+    g = torch.Generator("cuda").manual_seed(3)
+
+    def normal(*shape):
+        return torch.randn(*shape, generator=g, device="cuda").half()
+
+    q, k, v = (normal(1, 2, 100, 64).requires_grad_(True) for _ in range(3))
+    k2, v2 = (normal(1, 2, 40, 64).requires_grad_(True) for _ in range(2))
+    o = flash_attn_func(q, k2, v2, B200(), True, 0.125)
+    with pytest.raises(NotImplementedError):
+        o.backward(torch.ones_like(o))
+    # dO as an expanded and as a transposed tensor gives the gradients of its contiguous copy
+    for call in (lambda: flash_attn_func(q, k, v, B200(), True, 0.125),
+                 lambda: RetNetAttnFunc(q, k, v, None, B200(), True, 0.125, torch.tensor([0.97, 0.99]))):
+        o = call()
+        for do in (normal(1, 2, 64, 100).transpose(2, 3), normal(1, 2, 1, 64).expand(1, 2, 100, 64)):
+            got = torch.autograd.grad(o, (q, k, v), do, retain_graph=True)
+            want = torch.autograd.grad(o, (q, k, v), do.contiguous(), retain_graph=True)
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
+    # inference mode and no_grad give the same output without a node
+    with torch.no_grad():
+        assert torch.equal(flash_attn_func(q, k, v, B200(), True, 0.125), flash_attn_func(q, k, v, B200(), True, 0.125))
+        assert flash_attn_func(q, k, v, B200(), True, 0.125).grad_fn is None
+    o1, lse = flash_attn_func(q, k, v, B200(), True, 0.125, True)
+    assert o1.requires_grad and not lse.requires_grad
