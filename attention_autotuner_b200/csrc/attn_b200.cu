@@ -61,7 +61,7 @@ int fa_fwd_dispatch(const FaFwdArgs& a, int dqk, cudaStream_t st, bool profile, 
       // and store them by TMA (the tuner's choice at d = 128 as well); the grid form keeps its ring of four
       if constexpr (Cfg::DQK == 128 && Cfg::NQ == 2 && Cfg::NSTAGE == 4) {
         using P = FaFwdConfig<128, Cfg::DV, 2, 3, Cfg::BF16>;
-        if (fa_fwd_picks_persistent<P>(a)) return fa_fwd_persist_launch<P>(a, st);
+        if (!fa_fwd_is_decode<P>(a) && fa_fwd_picks_persistent<P>(a)) return fa_fwd_persist_launch<P>(a, st);
       }
       return fa_fwd_launch_auto<Cfg>(a, st);
     };

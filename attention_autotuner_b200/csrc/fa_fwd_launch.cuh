@@ -7,6 +7,7 @@
 
 #include <stdlib.h>
 
+#include "fa_decode_sm100.cuh"
 #include "fa_fwd_pair_sm100.cuh"
 #include "fa_fwd_persist_sm100.cuh"
 #include "fa_fwd_sm100.cuh"
@@ -119,6 +120,65 @@ int fa_fwd_persist_launch(const FaFwdArgs& a, cudaStream_t stream) {
   return check_launch("fa_fwd launch");
 }
 
+// Launcher of the decoding kernel (up to 16 query rows, head dimensions 64 and 128, the same for q, k and v).
+// nsplit = CTAs (a cluster) per slice; 0: chosen here: as many as keep all CTAs resident at once (two per SM) with at least
+// two blocks each. Measured at d = 128, 1 / 2 / 4 / 8 / 16 CTAs: BH = 32, Lkv = 16384: 117 / 65 / 45.1 / 45.2 / 53.6 us;
+// BH = 64, Lkv = 8192: 64.6 / 45.1 / 44.4 / 47.2 / 59.5; BH = 256, Lkv = 4096: 80.0 / 79.9 / 82.8 / 91 / 143. Clusters of
+// 16 are slower to place (BH = 16, Lkv = 32768: 46.9 us with 8, 56.0 with 16) and pay only where 8 leave half of the SMs
+// idle (BH = 4, Lkv = 32768: 34.7 and 22.6 us).
+inline int fa_decode_split(int BH, int nblk) {
+  int c = 1;
+  while (c < 8 && 2 * c * BH <= 296 && 2 * c <= nblk / 2) c *= 2;
+  return c == 8 && 16 * BH <= 148 && nblk >= 32 ? 16 : c;
+}
+
+template <int D, bool BF16>
+int fa_decode_launch(const FaFwdArgs& a, cudaStream_t stream, int nsplit = 0) {
+  using Cfg = FaDecodeConfig<D, BF16>;
+  if (!a.q || !a.k || !a.v || !a.o) return fail(kErrInvalidArgument, "fa_fwd: null tensor pointer");
+  if (a.BH <= 0 || a.Lq <= 0 || a.Lkv <= 0) return fail(kErrInvalidArgument, "fa_fwd: sizes must be positive");
+  if (a.BH > 65535) return fail(kErrInvalidArgument, "fa_fwd: batch*heads %d exceeds 65535", a.BH);
+  if (a.dv != D || a.Lq > Cfg::MAX_ROWS) return fail(kErrUnsupported, "fa_fwd: not a decoding shape");
+  if (!(a.scale > 0.f) || !isfinite(a.scale)) return fail(kErrInvalidArgument, "fa_fwd: scale must be positive and finite");
+  if (!aligned16(a.q) || !aligned16(a.k) || !aligned16(a.v) || !aligned32(a.o))
+    return fail(kErrInvalidArgument, "fa_fwd: inputs must be 16-byte aligned and the output 32-byte aligned");
+  CUtensorMap tk, tv;
+  int rc;
+  if ((rc = check_prior_status("fa_fwd"))) return rc;
+  if ((rc = bind_device_of(a.q, "fa_fwd"))) return rc;
+  if ((rc = make_tmap_3d(&tk, a.k, BF16, D, a.Lkv, a.BH, 64, Cfg::BN))) return rc;
+  if ((rc = make_tmap_3d(&tv, a.v, BF16, D, a.Lkv, a.BH, 64, Cfg::BN))) return rc;
+  FaFwdParams p;
+  p.o = a.o;
+  p.lse = a.lse;
+  p.dv_total = D;
+  p.Lq = a.Lq;
+  p.Lkv = a.Lkv;
+  p.causal = a.causal ? 1 : 0;
+  p.scale = a.scale;
+  p.scale_log2 = a.scale * 1.4426950408889634f;
+  auto kernel = &fa_decode_sm100_kernel<Cfg>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return fail(kErrCuda, "fa_fwd: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  const int c = nsplit > 0 ? nsplit : fa_decode_split(a.BH, (a.Lkv + Cfg::BN - 1) / Cfg::BN);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(c, 1, a.BH);
+  cfg.blockDim = dim3(Cfg::NTHREADS, 1, 1);
+  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = c;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, kernel, tk, tv, a.q, p);
+  if (e != cudaSuccess) return fail(kErrCuda, "fa_fwd: %s", cudaGetErrorString(e));
+  return check_launch("fa_fwd launch");
+}
+
 // The default tile (two query tiles, up to 128 V columns, no softmax variant) exists in both forms; the persistent one
 // runs where a CTA's work items are short, because what it saves lies at their boundaries. Measured against the grid
 // form in one session (d = 128, back-to-back launches), without a mask / under a causal one: 148 slices of L = 2048
@@ -136,8 +196,18 @@ bool fa_fwd_picks_persistent(const FaFwdArgs& a) {
   return false;
 }
 
+// Up to 16 query rows with one head dimension of 64 or 128: faster at every size measured (BH 1 to 512, Lkv 256 to 32768),
+// since the large tile works on 256 rows whatever it is given. The tile's row count is the limit.
+template <class Cfg>
+bool fa_fwd_is_decode(const FaFwdArgs& a) {
+  return (Cfg::DQK == 64 || Cfg::DQK == 128) && a.dv == Cfg::DQK && a.Lq <= 16 && fa_fwd_form_requested() == 0;
+}
+
 template <class Cfg>
 int fa_fwd_launch_auto(const FaFwdArgs& a, cudaStream_t stream) {
+  if constexpr (Cfg::DQK == 64 || Cfg::DQK == 128) {
+    if (fa_fwd_is_decode<Cfg>(a)) return fa_decode_launch<Cfg::DQK, Cfg::BF16>(a, stream);
+  }
   if constexpr (Cfg::NQ == 2 && Cfg::SPLIT == 1 && Cfg::NMMA == 1 && Cfg::EXP_EMU == 0 && Cfg::EXP_H2 == 0 && Cfg::DV <= 128) {
     if (fa_fwd_picks_persistent<Cfg>(a)) return fa_fwd_persist_launch<Cfg>(a, stream);
   }

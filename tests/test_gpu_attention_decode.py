@@ -1,0 +1,61 @@
+"""Attention forward with up to 16 query rows (csrc/fa_decode_sm100.cuh): every cluster size of the split over the keys,
+ragged last blocks, rows without a visible key, against the CPU fp32 oracle and against the large-tile kernel.
+
+Tolerances as in test_gpu_attention.py (the arithmetic is the same: P rounded to the storage type, fp32 elsewhere)."""
+import pytest
+import torch
+
+from attention_autotuner_b200.arch import B200
+from attention_autotuner_b200.ops.attention_interface import flash_attn_func
+from oracle import oracle
+from test_gpu_attention import check, rand_qkv, run_capi
+
+pytestmark = pytest.mark.gpu
+
+DT = {"fp16": torch.float16, "bf16": torch.bfloat16}
+
+# B, H, Lq, Lkv: cluster sizes 1 (many slices, or too few keys to split), 2, 4, 8, 16; one key; one short of, exactly and
+# one past a block of 64 / 128 keys; more rows than keys (rows that see nothing under the causal mask); the last row count
+SHAPES = [(1, 2, 1, 1), (1, 2, 16, 5), (1, 3, 3, 63), (2, 1, 16, 64), (1, 2, 8, 129), (2, 80, 1, 300), (3, 40, 2, 520),
+          (10, 5, 4, 1030), (3, 10, 1, 2049), (1, 2, 9, 4160), (1, 1, 16, 2176)]
+
+
+@pytest.mark.parametrize("dtype_name", ["fp16", "bf16"])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("d", [64, 128])
+def test_small_query_counts(lib, monkeypatch, dtype_name, causal, d):
+    for i, (B, H, Lq, Lkv) in enumerate(SHAPES):
+        q, k, v = rand_qkv(100 + i, B, H, Lq, Lkv, d, d, DT[dtype_name])
+        o, lse = run_capi(lib, q, k, v, d ** -0.5, causal)
+        oref, lref = oracle.attention_fwd(q, k, v, d ** -0.5, causal)
+        oref = torch.where(torch.isfinite(lref)[..., None], oref, torch.zeros(()))  # a row that sees no key: zeros
+        st = oracle.error_stats(o, oref)
+        assert oracle.within(st, dtype_name, scale_by_peak=True), ((B, H, Lq, Lkv), st)
+        fin = torch.isfinite(lref)
+        assert torch.equal(torch.isfinite(lse), fin) and (lse[fin] - lref[fin]).abs().max().item() < 1e-3
+        # the large tile on the same inputs (17 rows and more always take it)
+        monkeypatch.setenv("ATTN_B200_FA_FWD_FORM", "grid")
+        o2, _ = run_capi(lib, q, k, v, d ** -0.5, causal)
+        monkeypatch.delenv("ATTN_B200_FA_FWD_FORM")
+        # two roundings of P and one of O apart, relative to the peak
+        assert (o.float() - o2.float()).abs().max().item() <= (4 if dtype_name == "fp16" else 32) * 2.0 ** -10 * max(1.0, o2.abs().max().item())
+
+
+def test_first_row_count_of_the_large_tile(lib):
+    q, k, v = rand_qkv(5, 2, 2, 17, 700, 128, 128, torch.float16)
+    o, lse = run_capi(lib, q, k, v, 128 ** -0.5, True)
+    check(o, lse, q, k, v, 128 ** -0.5, True, "fp16")
+
+
+def test_operator_takes_strided_views_and_growing_peaks(lib):
+    """A decoding step reads a slice of a preallocated cache; scores that grow along the keys rescale at every block."""
+    g = torch.Generator().manual_seed(3)
+    cache_k = torch.randn(2, 4, 1024, 128, generator=g).half()
+    cache_v = torch.randn(2, 4, 1024, 128, generator=g).half()
+    q = torch.randn(2, 4, 1, 128, generator=g).half()
+    k = cache_k * torch.linspace(0.1, 3.0, 1024).half()[None, None, :, None]
+    n = 901
+    o, lse = flash_attn_func(q.cuda(), k.cuda()[:, :, :n], cache_v.cuda()[:, :, :n], B200(), True, 128 ** -0.5, return_lse=True)
+    oref, lref = oracle.attention_fwd(q, k[:, :, :n], cache_v[:, :, :n], 128 ** -0.5, True)
+    assert oracle.within(oracle.error_stats(o.cpu(), oref), "fp16", scale_by_peak=True)
+    assert (lse.cpu() - lref).abs().max().item() < 1e-3
