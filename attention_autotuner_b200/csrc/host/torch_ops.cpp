@@ -302,8 +302,12 @@ struct RetNode : public torch::autograd::Function<RetNode> {
 };
 
 // ------------------------------------------------------------------------------------------------ Python functions
+// Whether the call has to go through an autograd node. Forward-mode duals do too, whatever the grad mode: the node raises
+// (there is no jvp), whereas the plain launch would drop the tangents.
 bool any_grad(const Tensor& a, const Tensor& b, const Tensor& c) {
-  return at::GradMode::is_enabled() && (a.requires_grad() || b.requires_grad() || c.requires_grad());
+  for (const Tensor* t : {&a, &b, &c})
+    if (t->_fw_grad(/*level=*/0).defined() || (at::GradMode::is_enabled() && t->requires_grad())) return true;
+  return false;
 }
 // A tensor argument, or an undefined tensor for None; false for any other object.
 bool take_tensor(PyObject* obj, Tensor& t, bool none_ok = false) {

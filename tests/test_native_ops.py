@@ -73,3 +73,18 @@ def test_backward_errors_keep_their_class_and_strided_gradients_are_taken():
         assert flash_attn_func(q, k, v, B200(), True, 0.125).grad_fn is None
     o1, lse = flash_attn_func(q, k, v, B200(), True, 0.125, True)
     assert o1.requires_grad and not lse.requires_grad
+
+
+@pytest.mark.gpu
+def test_forward_mode_duals_are_refused_not_dropped():
+    import torch.autograd.forward_ad as fwAD
+    from attention_autotuner_b200.arch import B200
+    from attention_autotuner_b200.ops.attention_interface import flash_attn_func
+    from attention_autotuner_b200.ops.retnet_interface import RetNetAttnFunc
+    q, k, v, t = (torch.randn(1, 2, 64, 64, device="cuda").half() for _ in range(4))
+    with fwAD.dual_level(), torch.no_grad():
+        d = fwAD.make_dual(q, t)
+        with pytest.raises(RuntimeError):
+            flash_attn_func(d, k, v, B200(), True, 0.125)
+        with pytest.raises(RuntimeError):
+            RetNetAttnFunc(k, d, v, None, B200(), True, 0.125, torch.tensor([0.97, 0.99]))
