@@ -70,11 +70,6 @@ __device__ __forceinline__ void mma_m16n8k16(float* c, const uint32_t* a, uint32
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
   }
 }
-__device__ __forceinline__ float ld_shared_cluster_f32(uint32_t cluster_addr) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
-  return v;
-}
 
 // grid (cluster size, 1, BH), cluster (cluster size, 1, 1): CTA x of a slice takes every cluster-size-th share of the blocks.
 template <class Cfg>

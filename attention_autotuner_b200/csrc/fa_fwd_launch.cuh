@@ -27,7 +27,7 @@ struct FaFwdArgs {
 };
 
 template <class Cfg>
-int fa_fwd_launch(const FaFwdArgs& a, cudaStream_t stream) {
+int fa_fwd_launch(const FaFwdArgs& a, cudaStream_t stream, int nsplit = 1) {
   if (!a.q || !a.k || !a.v || !a.o) return fail(kErrInvalidArgument, "fa_fwd: null tensor pointer");
   if (a.BH <= 0 || a.Lq <= 0 || a.Lkv <= 0) return fail(kErrInvalidArgument, "fa_fwd: sizes must be positive");
   if (a.BH > 65535) return fail(kErrInvalidArgument, "fa_fwd: batch*heads %d exceeds 65535", a.BH);
@@ -58,7 +58,24 @@ int fa_fwd_launch(const FaFwdArgs& a, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
   if (e != cudaSuccess) return fail(kErrCuda, "fa_fwd: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   dim3 grid((a.Lq + Cfg::BM * Cfg::NQ - 1) / (Cfg::BM * Cfg::NQ), a.dv / Cfg::DV, a.BH);
-  kernel<<<grid, Cfg::NTHREADS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, p);
+  if constexpr (Cfg::KV_SPLIT) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid.x * nsplit, grid.y, grid.z);
+    cfg.blockDim = dim3(Cfg::NTHREADS, 1, 1);
+    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = nsplit;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, kernel, tq, tk, tv, p);
+    if (e != cudaSuccess) return fail(kErrCuda, "fa_fwd: %s", cudaGetErrorString(e));
+  } else {
+    kernel<<<grid, Cfg::NTHREADS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, p);
+  }
   return check_launch("fa_fwd launch");
 }
 
@@ -70,6 +87,13 @@ inline int fa_fwd_form_requested() {  // 0: automatic, 1: grid, 2: persistent
   if (s[0] == 'g') return 1;
   if (s[0] == 'p') return 2;
   return 0;
+}
+
+inline int sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+    return 148;
+  return sms;
 }
 
 // Launcher of the persistent kernel: one CTA per SM (fewer when there is less work) walking the work list.
@@ -112,9 +136,7 @@ int fa_fwd_persist_launch(const FaFwdArgs& a, cudaStream_t stream) {
   auto kernel = &fa_fwd_persist_sm100_kernel<Cfg>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::SMEM_BYTES);
   if (e != cudaSuccess) return fail(kErrCuda, "fa_fwd: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    sms = 148;
+  const int sms = sm_count();
   const int grid = pp.n_super < sms ? pp.n_super : sms;
   kernel<<<grid, Cfg::NTHREADS, Lay::SMEM_BYTES, stream>>>(tq, tk, tv, to, pp);
   return check_launch("fa_fwd launch");
@@ -184,14 +206,17 @@ int fa_decode_launch(const FaFwdArgs& a, cudaStream_t stream, int nsplit = 0) {
 // form in one session (d = 128, back-to-back launches), without a mask / under a causal one: 148 slices of L = 2048
 // +5 % / +18 %, B=8 H=16 L=4096 +1 % / +8 %, L = 8192 0 % / +3 %, B=16 H=32 L=16384 -2 % / -2 %, Lq=1024 x Lkv=16384
 // -3 % (with long items a static work list loses more to the slowest SM than the boundaries cost). The rule: persistent
-// up to 40 KV blocks per item on average (half of the blocks count under a causal mask).
+// up to 40 KV blocks per item on average (half of the blocks count under a causal mask). Where every item can have an SM of
+// its own there are no boundaries to save, and the work list's pairs would put two items on one SM: grid form (B=2 H=4
+// L=512 d=64: 12.3 against 19.1 us).
 template <class Cfg>
 bool fa_fwd_picks_persistent(const FaFwdArgs& a) {
   if constexpr (Cfg::NQ == 2 && Cfg::SPLIT == 1 && Cfg::NMMA == 1 && Cfg::EXP_EMU == 0 && Cfg::EXP_H2 == 0 && Cfg::DV <= 128) {
     const int form = fa_fwd_form_requested();
     const int nblk = (a.Lkv + Cfg::BN - 1) / Cfg::BN;
     const int avg_blocks = a.causal ? (nblk + 1) / 2 : nblk;
-    return form == 2 || (form == 0 && avg_blocks <= 40);
+    const long long items = static_cast<long long>(a.BH) * (a.dv / Cfg::DV) * ((a.Lq + 2 * Cfg::BM - 1) / (2 * Cfg::BM));
+    return form == 2 || (form == 0 && avg_blocks <= 40 && items > sm_count());
   }
   return false;
 }
@@ -203,12 +228,29 @@ bool fa_fwd_is_decode(const FaFwdArgs& a) {
   return (Cfg::DQK == 64 || Cfg::DQK == 128) && a.dv == Cfg::DQK && a.Lq <= 16 && fa_fwd_form_requested() == 0;
 }
 
+// CTAs per work item: the KV blocks of an item are split (FaFwdSplitConfig) while the parts all fit on the chip at once and
+// the item gets shorter by five blocks or more (the combination costs what three or four blocks take: B=1 H=16 L=1024 causal,
+// 8 blocks in two halves: 22.9 us against 22.6 whole; B=2 H=4 L=512 d=64, 4 blocks in four: 16.5 against 12.3).
+// Measured split / whole (grid form), bf16, causal: B=1 H=8 Lq=219 Lkv=2964 d=128 23.4 / 53.3 us; B=1 H=16 Lq=32 Lkv=10000
+// d=128 51 / 143; B=4 H=16 Lq=64 Lkv=4000 d=64 32.8 / 53.4; B=1 H=1 L=2048 d=128 22.5 / 36.9; B=1 H=4 Lq=1000 Lkv=9000 69 / 141.
+template <class Cfg>
+int fa_fwd_kv_split(const FaFwdArgs& a) {
+  if (fa_fwd_form_requested() != 0) return 1;
+  const long long items = static_cast<long long>(a.BH) * (a.dv / Cfg::DV) * ((a.Lq + 2 * Cfg::BM - 1) / (2 * Cfg::BM));
+  const int nblk = (a.Lkv + Cfg::BN - 1) / Cfg::BN, sms = sm_count();
+  int c = 1;
+  while (c < 8 && 2 * c * items <= sms && 2 * c <= nblk) c *= 2;
+  return nblk - (nblk + c - 1) / c >= 5 ? c : 1;
+}
+
 template <class Cfg>
 int fa_fwd_launch_auto(const FaFwdArgs& a, cudaStream_t stream) {
   if constexpr (Cfg::DQK == 64 || Cfg::DQK == 128) {
     if (fa_fwd_is_decode<Cfg>(a)) return fa_decode_launch<Cfg::DQK, Cfg::BF16>(a, stream);
   }
   if constexpr (Cfg::NQ == 2 && Cfg::SPLIT == 1 && Cfg::NMMA == 1 && Cfg::EXP_EMU == 0 && Cfg::EXP_H2 == 0 && Cfg::DV <= 128) {
+    const int nsplit = fa_fwd_kv_split<Cfg>(a);
+    if (nsplit > 1) return fa_fwd_launch<FaFwdSplitConfig<Cfg>>(a, stream, nsplit);
     if (fa_fwd_picks_persistent<Cfg>(a)) return fa_fwd_persist_launch<Cfg>(a, stream);
   }
   return fa_fwd_launch<Cfg>(a, stream);
