@@ -5,6 +5,7 @@
 #pragma once
 
 #include "ptx.cuh"
+#include "work_order.cuh"
 
 namespace ab200 {
 
@@ -21,10 +22,8 @@ struct ChainParams {
   int H, Lq, Lkv;
   float scale;
   int skip_upper;        // 1: blocks strictly above the diagonal are all zero and are skipped
-  // work list of the persistent grid: item w = (bh * ny + chunk) * nrb + row-block index
-  int nrb;               // 128-row blocks on the row side
+  WorkList work;         // row blocks (128 rows; 256 for CTA pairs) of slices bh * ny + chunk
   int ny;                // column chunks of the output (n2_total / N2)
-  int total_items;       // nrb * ny * BH
 };
 
 // One unit of work of the persistent chain kernel: a 128-row tile x one output-column chunk of one slice.

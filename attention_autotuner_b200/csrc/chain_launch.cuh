@@ -51,17 +51,17 @@ inline int ret_check_common(const RetArgs& a, const char* what) {
   return check_prior_status(what);
 }
 
-// CTAs of the persistent grid: one per SM (a CTA uses all of shared and tensor memory). The kernels hand out
-// equal-cost pairs of row blocks round-robin, so any grid size is balanced.
-inline int persistent_grid(int n_super) {
+// Workers of the persistent grid: one CTA per SM (a CTA uses all of shared and tensor memory).
+inline int persistent_workers() {
   static int sms = [] {
     int dev = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       n = 148;
     return n > 0 ? n : 148;
   }();
-  return n_super < sms ? n_super : sms;
+  return sms;
 }
+inline int persistent_grid(int units) { return units < persistent_workers() ? units : persistent_workers(); }
 
 // Launch helper: `overlap` marks the kernel as a programmatic dependent of the previous kernel in the stream (it may
 // start while that one drains; the kernels wait for it before they complete).
@@ -98,13 +98,11 @@ int chain_launch(const void* R, int r_len, const void* C, int c_len, const void*
   auto kernel = &chain_sm100_kernel<Cfg>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
   if (e != cudaSuccess) return fail(kErrCuda, "%s: cudaFuncSetAttribute: %s", what, cudaGetErrorString(e));
-  p.nrb = (r_len + 127) / 128;
+  const int nrb = (r_len + 127) / 128, workers = persistent_workers();
   p.ny = n2_total / Cfg::N2;
-  const long long total = static_cast<long long>(p.nrb) * p.ny * BH;
-  if (total > 0x7fffffffLL) return fail(kErrInvalidArgument, "%s: too many tiles", what);
-  p.total_items = static_cast<int>(total);
-  e = launch_maybe_overlapped(kernel, persistent_grid((p.total_items / p.nrb) * ((p.nrb + 1) / 2)), Cfg::NTHREADS,
-                              Cfg::SMEM_BYTES, stream, overlap, tr, tc, tt, p);
+  if (static_cast<long long>(nrb) * p.ny * BH > 0x3fffffffLL) return fail(kErrInvalidArgument, "%s: too many tiles", what);
+  p.work = make_work_list(BH * p.ny, nrb, workers, p.skip_upper != 0, 2.0 * c_len * (Cfg::K1 + Cfg::N2));
+  e = launch_maybe_overlapped(kernel, persistent_grid(p.work.units), Cfg::NTHREADS, Cfg::SMEM_BYTES, stream, overlap, tr, tc, tt, p);
   if (e != cudaSuccess) return fail(kErrCuda, "%s: %s", what, cudaGetErrorString(e));
   return check_launch(what);
 }
@@ -150,14 +148,11 @@ int chain_pair_launch(const void* R, int r_len, const void* C, int c_len, const 
     }
     max_clusters = n;
   }
-  p.nrb = (r_len + 255) / 256;
+  const int nrb = (r_len + 255) / 256;
   p.ny = n2_total / Cfg::N2;
-  const long long total = static_cast<long long>(p.nrb) * p.ny * BH;
-  if (total > 0x7fffffffLL) return fail(kErrInvalidArgument, "%s: too many tiles", what);
-  p.total_items = static_cast<int>(total);
-  // equal-cost super-items (pairs of row blocks) are handed out round-robin: any number of clusters is balanced
-  const int n_super = (p.total_items / p.nrb) * ((p.nrb + 1) / 2);
-  const int clusters = n_super < max_clusters ? n_super : max_clusters;
+  if (static_cast<long long>(nrb) * p.ny * BH > 0x3fffffffLL) return fail(kErrInvalidArgument, "%s: too many tiles", what);
+  p.work = make_work_list(BH * p.ny, nrb, max_clusters, p.skip_upper != 0, 2.0 * c_len * (Cfg::K1 + Cfg::N2));
+  const int clusters = p.work.units < max_clusters ? p.work.units : max_clusters;
   e = launch_maybe_overlapped(kernel, 2 * clusters, Cfg::NTHREADS, Cfg::SMEM_BYTES, stream, overlap, tr, tc, tt, to, p);
   if (e != cudaSuccess) return fail(kErrCuda, "%s: %s", what, cudaGetErrorString(e));
   return check_launch(what);

@@ -102,18 +102,16 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
   const uint32_t rank = cluster_ctarank();
   const int cluster_id = blockIdx.x >> 1;
   const int n_clusters = gridDim.x >> 1;
-  // Items are numbered  w = (bh * ny + chunk) * nrb + k,  256-row block = k-th heaviest  (nrb counts 256-row blocks
-  // here); see decode_step below for the order in which a cluster of the persistent grid takes them.
+  // An item is the k-th heaviest 256-row block of slice bh * ny + chunk; work_order.cuh has the order in which the
+  // clusters of the persistent grid take them.
   const int rows_len = (MODE == kChainRowK) ? p.Lkv : p.Lq;
   const int cols_len = (MODE == kChainRowK) ? p.Lq : p.Lkv;
   const int ncb = (cols_len + 127) / 128;
-  auto decode = [&](int w) -> ChainItem {
+  auto decode = [&](int k, int slice) -> ChainItem {
     ChainItem it;
-    const int k = w % p.nrb;
-    const int rest = w / p.nrb;
-    it.n_off = (rest % p.ny) * N2;
-    it.bh = rest / p.ny;
-    const int rb = (p.skip_upper && MODE != kChainRowK) ? (p.nrb - 1 - k) : k;
+    it.n_off = (slice % p.ny) * N2;
+    it.bh = slice / p.ny;
+    const int rb = (p.skip_upper && MODE != kChainRowK) ? (p.work.nrb - 1 - k) : k;
     it.row0 = rb * 256;  // first row of the pair; this CTA owns [row0 + rank*128, +128)
     it.t_start = 0;
     it.n_iter = ncb;
@@ -128,21 +126,11 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
     }
     return it;
   };
-  // Work list of a cluster. With the blocks above the diagonal skipped the k-th heaviest and the k-th lightest row
-  // block of a slice together always cost the same number of blocks, so the list is made of such pairs
-  // ("super-items", heavy one first) and handed out round-robin: every cluster gets the same work up to one
-  // super-item, whatever the number of clusters. (Single items handed out round-robin left the most loaded cluster
-  // about 10 % above the mean at 2048 rows.) Step u of a cluster: super-item s = cluster + n_clusters * (u / 2),
-  // first or second member.
-  const int npair = (p.nrb + 1) / 2;
-  const int n_super = (p.total_items / p.nrb) * npair;
-  const int n_steps = cluster_id < n_super ? 2 * ((n_super - cluster_id + n_clusters - 1) / n_clusters) : 0;
+  const int n_steps = p.work.steps(n_clusters);
   auto decode_step = [&](int u, ChainItem& it) -> bool {
-    const int sidx = cluster_id + n_clusters * (u >> 1);
-    const int j = sidx % npair;
-    const int k = (u & 1) ? p.nrb - 1 - j : j;
-    if ((u & 1) && k == j) return false;  // the middle row block of an odd count is its own partner
-    it = decode((sidx / npair) * p.nrb + k);
+    int k, slice;
+    if (!p.work.step(u, cluster_id, n_clusters, k, slice)) return false;
+    it = decode(k, slice);
     return true;
   };
 

@@ -98,23 +98,20 @@ chain_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constan
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // provably warp-uniform
   const int lane = threadIdx.x & 31;
-  // Persistent grid. Items are numbered  w = (bh * ny + chunk) * nrb + k,  row block = k-th heaviest, and taken in
-  // an order (decode_step below) in which the CTAs running at any moment cover a few neighbouring slices
-  // (operands shared in L2).
+  // Persistent grid. An item is the k-th heaviest row block of slice bh * ny + chunk; work_order.cuh has the order in
+  // which the CTAs take them.
   // Loads, MMAs and element-wise work of consecutive items overlap: the producer prefetches the next item's
   // resident tile as soon as GEMM1 of the current one has finished (r_free), the epilogue of an item runs
   // while GEMM1 of the next one is already in flight, and only the first GEMM2 waits for it (acc_free).
   const int rows_len = (MODE == kChainRowK) ? p.Lkv : p.Lq;
   const int cols_len = (MODE == kChainRowK) ? p.Lq : p.Lkv;
   const int ncb = (cols_len + 127) / 128;
-  auto decode = [&](int w) -> ChainItem {
+  auto decode = [&](int k, int slice) -> ChainItem {
     ChainItem it;
-    const int k = w % p.nrb;
-    const int rest = w / p.nrb;
-    it.n_off = (rest % p.ny) * N2;
-    it.bh = rest / p.ny;
+    it.n_off = (slice % p.ny) * N2;
+    it.bh = slice / p.ny;
     // heaviest row blocks first when blocks are skipped (Fwd/RowQ: late queries; RowK: early keys)
-    const int rb = (p.skip_upper && MODE != kChainRowK) ? (p.nrb - 1 - k) : k;
+    const int rb = (p.skip_upper && MODE != kChainRowK) ? (p.work.nrb - 1 - k) : k;
     it.row0 = rb * 128;
     it.t_start = 0;
     it.n_iter = ncb;
@@ -129,20 +126,11 @@ chain_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constan
     }
     return it;
   };
-  // Work list of a CTA. With the blocks above the diagonal skipped the k-th heaviest and the k-th lightest row
-  // block of a slice together always cost the same number of blocks, so the list is made of such pairs
-  // ("super-items", heavy one first) and handed out round-robin: every CTA gets the same work up to one
-  // super-item, whatever the grid size. Step u of a CTA: super-item blockIdx.x + gridDim.x * (u / 2), first or
-  // second member.
-  const int npair = (p.nrb + 1) / 2;
-  const int n_super = (p.total_items / p.nrb) * npair;
-  const int n_steps = static_cast<int>(blockIdx.x) < n_super ? 2 * ((n_super - blockIdx.x + gridDim.x - 1) / gridDim.x) : 0;
+  const int n_steps = p.work.steps(gridDim.x);
   auto decode_step = [&](int u, ChainItem& it) -> bool {
-    const int sidx = blockIdx.x + gridDim.x * (u >> 1);
-    const int j = sidx % npair;
-    const int k = (u & 1) ? p.nrb - 1 - j : j;
-    if ((u & 1) && k == j) return false;  // the middle row block of an odd count is its own partner
-    it = decode((sidx / npair) * p.nrb + k);
+    int k, slice;
+    if (!p.work.step(u, blockIdx.x, gridDim.x, k, slice)) return false;
+    it = decode(k, slice);
     return true;
   };
 
