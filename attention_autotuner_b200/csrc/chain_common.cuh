@@ -192,27 +192,6 @@ __device__ __forceinline__ void chain_mask_prefetch_t(const ChainParams& p, int 
   }
 }
 
-// out[h][j][i] = in[h][i][j] for a 16-bit tensor in [H, rows, cols]: 32 x 32 tiles through shared memory (padded rows,
-// no bank conflicts), coalesced on both sides. grid = (ceil(cols / 32), ceil(rows / 32), H), block = (32, 8).
-__global__ void mask_transpose_kernel(const uint16_t* __restrict__ in, uint16_t* __restrict__ out, int rows, int cols) {
-  __shared__ uint16_t tile[32][34];
-  const size_t plane = static_cast<size_t>(rows) * cols;
-  const uint16_t* src = in + blockIdx.z * plane;
-  uint16_t* dst = out + blockIdx.z * plane;
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-#pragma unroll
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int r = r0 + i, c = c0 + threadIdx.x;
-    tile[i][threadIdx.x] = (r < rows && c < cols) ? src[static_cast<size_t>(r) * cols + c] : uint16_t(0);
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = threadIdx.y; i < 32; i += 8) {
-    const int c = c0 + i, r = r0 + threadIdx.x;  // out row = in column
-    if (c < cols && r < rows) dst[static_cast<size_t>(c) * rows + r] = tile[threadIdx.x][i];
-  }
-}
-
 // RowK flavours: thread (lane L of its warp) owns key grow0 + L and needs M[h][query][key] for the 64 queries of its
 // two chunks, i.e. a COLUMN of the mask. Reading it with 64 two-byte loads per thread and block cost 0.9 ms of the
 // 1.55 ms backward at config 4 (measured by replacing the loads with a constant). Here the warp reads its
@@ -239,6 +218,43 @@ __device__ __forceinline__ void chain_transpose8x8_b16(uint32_t (&r)[4], int lan
   r[1] = __byte_perm(z1, c0, odd ? 0x3276 : 0x7610);  // (row 2 | row 3)
   r[2] = __byte_perm(z2, c1, odd ? 0x3254 : 0x5410);  // (row 4 | row 5)
   r[3] = __byte_perm(z3, c1, odd ? 0x3276 : 0x7610);  // (row 6 | row 7)
+}
+
+// out[h][j][i] = in[h][i][j] for a 16-bit tensor in [H, rows, cols], rows and cols multiples of 8, both 16-byte aligned.
+// Bound by memory: 64 x 64 tiles, 16-byte loads (a group of 8 lanes takes an 8 x 8 block, one row per lane), the blocks
+// transposed in registers, and the tile turned in shared memory (16-byte pieces, swizzled) so that the stores are whole
+// rows of 128 bytes. H = 8, 2048 x 2048 (134 MB in and out): 31 us = 4.3 TB/s; with two-byte accesses and 32 x 32 tiles it was
+// 81. grid = (ceil(cols / 64), ceil(rows / 64), H), block = 256.
+__global__ void __launch_bounds__(256) mask_transpose_kernel(const uint16_t* __restrict__ in, uint16_t* __restrict__ out, int rows,
+                                                             int cols) {
+  __shared__ uint4 tile[64 * 8];  // [column][group of 8 rows, position ^ (column & 7)]
+  const size_t plane = static_cast<size_t>(rows) * cols;
+  const uint16_t* src = in + blockIdx.z * plane;
+  uint16_t* dst = out + blockIdx.z * plane;
+  const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row = r0 + warp * 8 + (lane & 7);
+  uint4 v[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int col = c0 + (h * 4 + (lane >> 3)) * 8;
+    v[h] = make_uint4(0, 0, 0, 0);
+    if (row < rows && col < cols) v[h] = __ldg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(row) * cols + col));
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t r[4] = {v[h].x, v[h].y, v[h].z, v[h].w};
+    chain_transpose8x8_b16(r, lane);
+    const int c = (h * 4 + (lane >> 3)) * 8 + (lane & 7);
+    tile[c * 8 + (warp ^ (c & 7))] = make_uint4(r[0], r[1], r[2], r[3]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = h * 256 + threadIdx.x, c = i >> 3, rg = i & 7;
+    if (c0 + c < cols && r0 + rg * 8 < rows)
+      *reinterpret_cast<uint4*>(dst + static_cast<size_t>(c0 + c) * rows + r0 + rg * 8) = tile[c * 8 + (rg ^ (c & 7))];
+  }
 }
 
 // grow0 = first key of the warp (a multiple of 32); all 32 lanes of the warp must call this together.

@@ -216,8 +216,8 @@ int ret_bwd_launch(const RetArgs& a, cudaStream_t stream) {
   const size_t mask_bytes = static_cast<size_t>(a.H) * a.Lq * a.Lkv * 2u;
   const uint16_t* mask_t = nullptr;
   if (a.mask && a.workspace && aligned16(a.workspace) && a.workspace_bytes >= mask_bytes && a.Lq % 8 == 0) {
-    dim3 tgrid((a.Lkv + 31) / 32, (a.Lq + 31) / 32, a.H);
-    mask_transpose_kernel<<<tgrid, dim3(32, 8, 1), 0, stream>>>(reinterpret_cast<const uint16_t*>(a.mask),
+    dim3 tgrid((a.Lkv + 63) / 64, (a.Lq + 63) / 64, a.H);
+    mask_transpose_kernel<<<tgrid, 256, 0, stream>>>(reinterpret_cast<const uint16_t*>(a.mask),
                                                               reinterpret_cast<uint16_t*>(a.workspace), a.Lq, a.Lkv);
     if ((rc = check_launch("ret_bwd mask transpose"))) return rc;
     mask_t = reinterpret_cast<const uint16_t*>(a.workspace);
