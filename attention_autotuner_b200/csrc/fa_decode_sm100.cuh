@@ -3,8 +3,7 @@
 // What bounds it: reading K and V once. 16 rows give 32 FLOP per byte of K and V, a tenth of what the tensor cores need to
 // be the limit, so the tile of 128 query rows of fa_fwd_sm100.cuh does nothing but fetch: one CTA per (batch, head) slice,
 // one block of 128 keys (64 KB) per 1.8 us of serial S -> softmax -> P V chain. Here
-//   * the keys of a slice are split over the CTAs of a thread-block cluster (1 to 16, chosen by the launcher so that the
-//     whole chip reads); each keeps its own maximum, sum and accumulator, and the cluster combines them through
+//   * the keys of a slice are split over the CTAs of a thread-block cluster (1, 4 or 8, by the number of keys); each keeps its own maximum, sum and accumulator, and the cluster combines them through
 //     distributed shared memory at the end: one launch, no scratch memory;
 //   * a CTA streams blocks of 64 keys (128 at d = 64; K and V together, 32 KB) by TMA through a ring of three, two CTAs
 //     per SM: 192 KB on the way per SM;
@@ -14,8 +13,8 @@
 // Same arithmetic as the large tiles: fp32 scores, maxima, sums and accumulators, P rounded to the storage type.
 //
 // Measured (B200, bf16, causal, cold caches, against the 256-row tile of one CTA per slice): BH = 32, Lq = 1, Lkv = 16384,
-// d = 128: 45 us = 5.95 TB/s against 230 us; d = 64: 26.5 us. BH = 4, Lkv = 32768, d = 128: 22.6 us against 450 us.
-// BH = 512, Lkv = 2048, d = 128: 80 us = 6.7 TB/s. Distance to 64-bit results 2.5e-4 / 2.1e-3 (fp16 / bf16, 2-norm), the
+// d = 128: 45 us = 5.95 TB/s against 230 us; d = 64: 26.5 us. BH = 1, Lkv = 32768, d = 128: 33 us against 450.
+// BH = 256, Lkv = 4096, d = 128: 83 us = 6.5 TB/s. Distance to 64-bit results 2.5e-4 / 2.1e-3 (fp16 / bf16, 2-norm), the
 // large tile 2.9e-4 / 2.4e-3: its running maximum may lag by 2^8, this one's does not.
 #pragma once
 

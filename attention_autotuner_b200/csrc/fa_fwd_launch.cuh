@@ -27,7 +27,7 @@ struct FaFwdArgs {
 };
 
 template <class Cfg>
-int fa_fwd_launch(const FaFwdArgs& a, cudaStream_t stream, int nsplit = 1) {
+int fa_fwd_launch(const FaFwdArgs& a, cudaStream_t stream) {
   if (!a.q || !a.k || !a.v || !a.o) return fail(kErrInvalidArgument, "fa_fwd: null tensor pointer");
   if (a.BH <= 0 || a.Lq <= 0 || a.Lkv <= 0) return fail(kErrInvalidArgument, "fa_fwd: sizes must be positive");
   if (a.BH > 65535) return fail(kErrInvalidArgument, "fa_fwd: batch*heads %d exceeds 65535", a.BH);
@@ -58,24 +58,7 @@ int fa_fwd_launch(const FaFwdArgs& a, cudaStream_t stream, int nsplit = 1) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
   if (e != cudaSuccess) return fail(kErrCuda, "fa_fwd: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   dim3 grid((a.Lq + Cfg::BM * Cfg::NQ - 1) / (Cfg::BM * Cfg::NQ), a.dv / Cfg::DV, a.BH);
-  if constexpr (Cfg::KV_SPLIT) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid.x * nsplit, grid.y, grid.z);
-    cfg.blockDim = dim3(Cfg::NTHREADS, 1, 1);
-    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = nsplit;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, kernel, tq, tk, tv, p);
-    if (e != cudaSuccess) return fail(kErrCuda, "fa_fwd: %s", cudaGetErrorString(e));
-  } else {
-    kernel<<<grid, Cfg::NTHREADS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, p);
-  }
+  kernel<<<grid, Cfg::NTHREADS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, p);
   return check_launch("fa_fwd launch");
 }
 
@@ -143,16 +126,13 @@ int fa_fwd_persist_launch(const FaFwdArgs& a, cudaStream_t stream) {
 }
 
 // Launcher of the decoding kernel (up to 16 query rows, head dimensions 64 and 128, the same for q, k and v).
-// nsplit = CTAs (a cluster) per slice; 0: chosen here: as many as keep all CTAs resident at once (two per SM) with at least
-// two blocks each. Measured at d = 128, 1 / 2 / 4 / 8 / 16 CTAs: BH = 32, Lkv = 16384: 117 / 65 / 45.1 / 45.2 / 53.6 us;
-// BH = 64, Lkv = 8192: 64.6 / 45.1 / 44.4 / 47.2 / 59.5; BH = 256, Lkv = 4096: 80.0 / 79.9 / 82.8 / 91 / 143. Clusters of
-// 16 are slower to place (BH = 16, Lkv = 32768: 46.9 us with 8, 56.0 with 16) and pay only where 8 leave half of the SMs
-// idle (BH = 4, Lkv = 32768: 34.7 and 22.6 us).
-inline int fa_decode_split(int BH, int nblk) {
-  int c = 1;
-  while (c < 8 && 2 * c * BH <= 296 && 2 * c <= nblk / 2) c *= 2;
-  return c == 8 && 16 * BH <= 148 && nblk >= 32 ? 16 : c;
-}
+// nsplit = CTAs (a cluster) per slice; 0: chosen here, by the number of blocks alone: the order in which a slice's partial
+// results are added, and so its output to the last bit, must not depend on how many other slices are in the launch
+// (sharding by slices gives the same bits on any number of ranks). Measured at d = 128, 1 / 4 / 8 CTAs: BH = 32, Lkv = 16384:
+// 117 / 45.1 / 45.2 us; BH = 16, Lkv = 32768: 223 / 65 / 46.9; BH = 64, Lkv = 8192: 64.6 / 44.6 / 47.2; BH = 256, Lkv = 4096:
+// 80.0 / 82.8 / 91; BH = 512, Lkv = 2048: 79.6 / 87 / 114, Lkv = 256: 18.5 / 36 / 70. Four lose little with many slices and
+// win most of what there is with few; eight where a cache is long enough to hide the larger cluster.
+inline int fa_decode_split(int nblk) { return nblk >= 256 ? 8 : nblk >= 32 ? 4 : 1; }
 
 template <int D, bool BF16>
 int fa_decode_launch(const FaFwdArgs& a, cudaStream_t stream, int nsplit = 0) {
@@ -181,9 +161,8 @@ int fa_decode_launch(const FaFwdArgs& a, cudaStream_t stream, int nsplit = 0) {
   p.scale_log2 = a.scale * 1.4426950408889634f;
   auto kernel = &fa_decode_sm100_kernel<Cfg>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return fail(kErrCuda, "fa_fwd: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  const int c = nsplit > 0 ? nsplit : fa_decode_split(a.BH, (a.Lkv + Cfg::BN - 1) / Cfg::BN);
+  const int c = nsplit > 0 ? nsplit : fa_decode_split((a.Lkv + Cfg::BN - 1) / Cfg::BN);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(c, 1, a.BH);
   cfg.blockDim = dim3(Cfg::NTHREADS, 1, 1);
@@ -228,29 +207,12 @@ bool fa_fwd_is_decode(const FaFwdArgs& a) {
   return (Cfg::DQK == 64 || Cfg::DQK == 128) && a.dv == Cfg::DQK && a.Lq <= 16 && fa_fwd_form_requested() == 0;
 }
 
-// CTAs per work item: the KV blocks of an item are split (FaFwdSplitConfig) while the parts all fit on the chip at once and
-// the item gets shorter by five blocks or more (the combination costs what three or four blocks take: B=1 H=16 L=1024 causal,
-// 8 blocks in two halves: 22.9 us against 22.6 whole; B=2 H=4 L=512 d=64, 4 blocks in four: 16.5 against 12.3).
-// Measured split / whole (grid form), bf16, causal: B=1 H=8 Lq=219 Lkv=2964 d=128 23.4 / 53.3 us; B=1 H=16 Lq=32 Lkv=10000
-// d=128 51 / 143; B=4 H=16 Lq=64 Lkv=4000 d=64 32.8 / 53.4; B=1 H=1 L=2048 d=128 22.5 / 36.9; B=1 H=4 Lq=1000 Lkv=9000 69 / 141.
-template <class Cfg>
-int fa_fwd_kv_split(const FaFwdArgs& a) {
-  if (fa_fwd_form_requested() != 0) return 1;
-  const long long items = static_cast<long long>(a.BH) * (a.dv / Cfg::DV) * ((a.Lq + 2 * Cfg::BM - 1) / (2 * Cfg::BM));
-  const int nblk = (a.Lkv + Cfg::BN - 1) / Cfg::BN, sms = sm_count();
-  int c = 1;
-  while (c < 8 && 2 * c * items <= sms && 2 * c <= nblk) c *= 2;
-  return nblk - (nblk + c - 1) / c >= 5 ? c : 1;
-}
-
 template <class Cfg>
 int fa_fwd_launch_auto(const FaFwdArgs& a, cudaStream_t stream) {
   if constexpr (Cfg::DQK == 64 || Cfg::DQK == 128) {
     if (fa_fwd_is_decode<Cfg>(a)) return fa_decode_launch<Cfg::DQK, Cfg::BF16>(a, stream);
   }
   if constexpr (Cfg::NQ == 2 && Cfg::SPLIT == 1 && Cfg::NMMA == 1 && Cfg::EXP_EMU == 0 && Cfg::EXP_H2 == 0 && Cfg::DV <= 128) {
-    const int nsplit = fa_fwd_kv_split<Cfg>(a);
-    if (nsplit > 1) return fa_fwd_launch<FaFwdSplitConfig<Cfg>>(a, stream, nsplit);
     if (fa_fwd_picks_persistent<Cfg>(a)) return fa_fwd_persist_launch<Cfg>(a, stream);
   }
   return fa_fwd_launch<Cfg>(a, stream);

@@ -21,7 +21,6 @@
 #pragma once
 
 #include "ptx.cuh"
-#include "ptx_pair.cuh"  // cluster barrier, distributed shared memory addresses
 
 namespace ab200 {
 
@@ -84,20 +83,6 @@ struct FaFwdConfig {
   static_assert(TMEM_COLS_USED <= 512, "TMEM overflow: NQ*(128+DV) must be <= 512 columns");
   static_assert(DV <= 256, "one PV MMA covers at most N=256");
   static_assert(SMEM_BYTES <= 232448, "shared memory overflow");
-  static constexpr bool KV_SPLIT = false;
-};
-
-// The same tile with the keys of a work item split over the CTAs of a cluster (grid x = query block * cluster size +
-// rank): for calls with far fewer work items than SMs, where the one CTA of an item walks its KV blocks one after another
-// (1.8 to 2.2 us each, S -> softmax -> P V) while most SMs are idle. Every CTA runs the kernel on its share of the blocks;
-// at the end the unnormalised tiles, maxima and sums are combined in fp32 through distributed shared memory (they take the
-// place of the operand tiles): no scratch memory, no second launch.
-template <class Base>
-struct FaFwdSplitConfig : Base {
-  static_assert(Base::NQ == 2 && Base::SPLIT == 1 && Base::NMMA == 1 && Base::EXP_EMU == 0 && Base::EXP_H2 == 0, "default tile");
-  static constexpr bool KV_SPLIT = true;
-  static constexpr int PART_O_BYTES = 2 * 128 * Base::DV * 4;  // [256 rows][DV], 16-byte pieces at position ^ (row & 7)
-  static_assert(PART_O_BYTES + 2 * 256 * 4 <= Base::SMEM_TILES, "the partial results live in the operand tiles");
 };
 
 // Optional event trace (compile with -DAB200_TRACE): CTA (0,0,0) records clock64() at the hand-off points of
@@ -147,14 +132,8 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   constexpr int NMMA = Cfg::NMMA;
   constexpr int kTmaWarp = 4 * NQ * SPLIT + NMMA;
 
-  uint32_t split_rank = 0, nsplit = 1;  // this CTA's share of the KV blocks
-  if constexpr (Cfg::KV_SPLIT) {
-    split_rank = cluster_ctarank();
-    nsplit = cluster_nctarank();
-  }
   // Heaviest (latest) query blocks first under a causal mask.
-  const int xblk = Cfg::KV_SPLIT ? blockIdx.x / nsplit : blockIdx.x, nxblk = Cfg::KV_SPLIT ? gridDim.x / nsplit : gridDim.x;
-  const int qblk = p.causal ? (nxblk - 1 - xblk) : xblk;
+  const int qblk = p.causal ? (gridDim.x - 1 - blockIdx.x) : blockIdx.x;
   // grid: x = query block, y = V-column chunk, z = (batch, head)
   const int bh = blockIdx.z;
   const int dv_off = blockIdx.y * DV;
@@ -175,14 +154,6 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (m_base + s * BM >= p.Lq) n = 0;  // tile entirely past the end of Q
     nblk[s] = n;
     nmax = n > nmax ? n : nmax;
-  }
-  int jb = 0;  // first KV block of this CTA; block numbers below count from it
-  if constexpr (Cfg::KV_SPLIT) {
-    jb = nmax * static_cast<int>(split_rank) / static_cast<int>(nsplit);
-    const int je = nmax * static_cast<int>(split_rank + 1) / static_cast<int>(nsplit);
-#pragma unroll
-    for (int s = 0; s < NQ; ++s) nblk[s] = min(max(nblk[s] - jb, 0), je - jb);
-    nmax = je - jb;
   }
 
   if (threadIdx.x == 0) {
@@ -249,11 +220,11 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if ((t & 1) == 0) {
           mbar_expect_tx(&kv_full[slot], Cfg::K_TILE_BYTES);
 #pragma unroll
-          for (int c = 0; c < DQK / 64; ++c) tma_load_3d(dst + c * (BN * 128), &tmK, &kv_full[slot], c * 64, (jb + j) * BN, bh);
+          for (int c = 0; c < DQK / 64; ++c) tma_load_3d(dst + c * (BN * 128), &tmK, &kv_full[slot], c * 64, j * BN, bh);
         } else {
           mbar_expect_tx(&kv_full[slot], Cfg::V_TILE_BYTES);
 #pragma unroll
-          for (int c = 0; c < DV / 64; ++c) tma_load_3d(dst + c * (BN * 128), &tmV, &kv_full[slot], dv_off + c * 64, (jb + j) * BN, bh);
+          for (int c = 0; c < DV / 64; ++c) tma_load_3d(dst + c * (BN * 128), &tmV, &kv_full[slot], dv_off + c * 64, j * BN, bh);
         }
         t_issued = t + 1;
         if (t == 0) {
@@ -380,11 +351,6 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
     }
   }
-  if constexpr (Cfg::KV_SPLIT) {  // the cluster barriers around the softmax warps' last step
-    __syncwarp();
-    cluster_sync();
-    cluster_sync();
-  }
   } else if constexpr (SPLIT == 2) {
     // ------------------------------------------------------------------ softmax warpgroups, two per query tile
 #include "fa_fwd_softmax_split.cuh"
@@ -420,7 +386,7 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tc_wait_ld();
       }
       if (threadIdx.x % 128 == 0) AB200_TR(s, j, 2);
-      const int n0 = (jb + j) * BN;
+      const int n0 = j * BN;
       // masking: keys past Lkv (ragged tail) and, under causal, keys j > i + shift
       const bool tail_blk = (n0 + BN > p.Lkv);
       const bool diag_blk = p.causal && (n0 + BN - 1 > m_base + s * BM + causal_shift);
@@ -526,80 +492,6 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (threadIdx.x % 128 == 0) AB200_TR(s, j, 5);
     }
 
-    if constexpr (Cfg::KV_SPLIT) {
-      // partial results into the operand tiles' memory, once both tiles' MMAs have read them (each warpgroup waits for its
-      // own, then for the other warpgroup; also after an aborted wait)
-      if (ok && n_my > 0) ok = mbar_wait_warp(&o_done[s], (n_my - 1) & 1, ab, kTagODone);
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      tc_fence_after();
-      const int prow = s * BM + row_in_tile;
-      uint8_t* po = smem + prow * (DV * 4);
-      float* pm = reinterpret_cast<float*>(smem + Cfg::PART_O_BYTES);
-      const bool have = ok && n_my > 0;
-      pm[prow] = have ? m_ref * p.scale_log2 : -INFINITY;  // exp2 units
-      pm[256 + prow] = have ? l_sum : 0.f;
-      if (have) {
-#pragma unroll
-        for (int c0 = 0; c0 < DV; c0 += 32) {
-          uint32_t r[32];
-          tmem_ld32(tO + c0, r);
-          tc_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 32; i += 4)
-            *reinterpret_cast<uint4*>(po + ((((c0 + i) >> 2) ^ (prow & 7)) << 4)) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
-        }
-      }
-      // the item's rows from the partial results of the whole cluster, every CTA a share of the rows: a softmax thread takes
-      // eight columns of one row (the other warps have given up their registers). All threads of all CTAs reach both cluster
-      // barriers, here or at the end of the other roles, also after an aborted wait.
-      __syncwarp();
-      cluster_sync();
-      constexpr int TPR = DV / 8;  // threads per row
-      const uint32_t a_o = smem_u32(smem), a_m = a_o + Cfg::PART_O_BYTES;
-      for (int i = threadIdx.x; i < (256 / static_cast<int>(nsplit)) * TPR; i += 256) {
-        const int prow = (i / TPR) * static_cast<int>(nsplit) + static_cast<int>(split_rank), c8 = i % TPR;
-        const int row = m_base + prow;
-        if (row >= p.Lq) continue;
-        // (unrolled over the largest cluster: one remote access takes several hundred cycles, so they are all in flight)
-        float mc[8], lc[8], x[8][8];
-#pragma unroll
-        for (uint32_t c = 0; c < 8; ++c) {
-          mc[c] = -INFINITY;
-          lc[c] = 0.f;
-          if (c < nsplit) {
-            const uint32_t base = mapa_shared(a_o, c);
-            mc[c] = ld_shared_cluster_f32(base + Cfg::PART_O_BYTES + 4 * prow);
-            lc[c] = ld_shared_cluster_f32(base + Cfg::PART_O_BYTES + 4 * (256 + prow));
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-              ld_shared_cluster_v4(base + prow * (DV * 4) + (((2 * c8 + h) ^ (prow & 7)) << 4), x[c] + 4 * h);
-          }
-        }
-        float m = mc[0];
-#pragma unroll
-        for (uint32_t c = 1; c < 8; ++c) m = fmaxf(m, mc[c]);
-        float acc[8] = {};
-        float l = 0.f;
-#pragma unroll
-        for (uint32_t c = 0; c < 8; ++c) {
-          if (mc[c] == -INFINITY) continue;  // no such CTA, or no visible key there: its rows were not written
-          const float f = ex2_approx(mc[c] - m);
-          l = fmaf(f, lc[c], l);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) acc[e] = fmaf(f, x[c][e], acc[e]);
-        }
-        const float inv_l = l > 0.f ? 1.0f / l : 0.f;
-        uint4 v;
-        v.x = pack2<BF16>(acc[0] * inv_l, acc[1] * inv_l);
-        v.y = pack2<BF16>(acc[2] * inv_l, acc[3] * inv_l);
-        v.z = pack2<BF16>(acc[4] * inv_l, acc[5] * inv_l);
-        v.w = pack2<BF16>(acc[6] * inv_l, acc[7] * inv_l);
-        const size_t orow = static_cast<size_t>(bh) * p.Lq + row;
-        *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.o) + orow * p.dv_total + dv_off + c8 * 8) = v;
-        if (p.lse != nullptr && dv_off == 0 && c8 == 0) p.lse[orow] = l > 0.f ? m * 0.6931471805599453f + __logf(l) : -INFINITY;
-      }
-      cluster_sync();  // no CTA leaves while another may still read its shared memory
-    } else
     // epilogue: O / l  ->  global, lse
     if (ok && n_my > 0) {
       ok = mbar_wait_warp(&o_done[s], (n_my - 1) & 1, ab, kTagODone);

@@ -16,19 +16,11 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ uint32_t cluster_nctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-// Loads from the shared memory of any CTA of the cluster (address from mapa_shared).
+// Load from the shared memory of any CTA of the cluster (address from mapa_shared).
 __device__ __forceinline__ float ld_shared_cluster_f32(uint32_t cluster_addr) {
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
   return v;
-}
-__device__ __forceinline__ void ld_shared_cluster_v4(uint32_t cluster_addr, float* v) {
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(cluster_addr) : "memory");
 }
 // Full barrier over all threads of the cluster (hardware barrier; every thread of both CTAs must reach it).
 __device__ __forceinline__ void cluster_sync() {

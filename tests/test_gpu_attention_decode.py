@@ -14,10 +14,11 @@ pytestmark = pytest.mark.gpu
 
 DT = {"fp16": torch.float16, "bf16": torch.bfloat16}
 
-# B, H, Lq, Lkv: cluster sizes 1 (many slices, or too few keys to split), 2, 4, 8, 16; one key; one short of, exactly and
-# one past a block of 64 / 128 keys; more rows than keys (rows that see nothing under the causal mask); the last row count
-SHAPES = [(1, 2, 1, 1), (1, 2, 16, 5), (1, 3, 3, 63), (2, 1, 16, 64), (1, 2, 8, 129), (2, 80, 1, 300), (3, 40, 2, 520),
-          (10, 5, 4, 1030), (3, 10, 1, 2049), (1, 2, 9, 4160), (1, 1, 16, 2176)]
+# B, H, Lq, Lkv: one key; one short of, exactly and one past a block (64 keys at d = 128, 128 at d = 64); more rows than
+# keys (rows that see nothing under the causal mask); the last row count; clusters of 1, of 4 (from 32 blocks) and of 8 (from
+# 256) at both head dimensions, with uneven shares
+SHAPES = [(1, 2, 1, 1), (1, 2, 16, 5), (1, 3, 3, 63), (2, 1, 16, 64), (1, 2, 8, 129), (2, 80, 1, 300), (3, 10, 1, 2049),
+          (1, 2, 9, 4160), (1, 1, 16, 2176), (1, 1, 2, 16385), (1, 1, 1, 32800)]
 
 
 @pytest.mark.parametrize("dtype_name", ["fp16", "bf16"])
@@ -59,3 +60,12 @@ def test_operator_takes_strided_views_and_growing_peaks(lib):
     oref, lref = oracle.attention_fwd(q, k[:, :, :n], cache_v[:, :, :n], 128 ** -0.5, True)
     assert oracle.within(oracle.error_stats(o.cpu(), oref), "fp16", scale_by_peak=True)
     assert (lse.cpu() - lref).abs().max().item() < 1e-3
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_a_slice_has_the_same_bits_in_any_launch(lib, d):
+    q, k, v = rand_qkv(11, 12, 1, 3, 5000, d, d, torch.bfloat16)
+    o, lse = run_capi(lib, q, k, v, d ** -0.5, True)
+    for n in (1, 5):
+        o1, lse1 = run_capi(lib, q[:n], k[:n], v[:n], d ** -0.5, True)
+        assert torch.equal(o1, o[:n]) and torch.equal(lse1, lse[:n])
