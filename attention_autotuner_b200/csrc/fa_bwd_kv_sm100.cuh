@@ -130,7 +130,7 @@ struct FaBwdKvConfig {
   static_assert(SMEM_BYTES <= 232448, "shared memory");
 };
 
-template <class Cfg>
+template <class Cfg, bool SINGLES = false>
 __global__ void __launch_bounds__(Cfg::NTHREADS, 1)
 fa_bwd_kv_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                        const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
@@ -184,7 +184,7 @@ fa_bwd_kv_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     it.row0 = rb * 128;
     it.t_start = 0;
     it.n_iter = ncb;
-    if (p.causal) {
+    if (!SINGLES && p.causal) {
       it.t_start = rb;  // query blocks before this key block see none of its keys
       it.n_iter = ncb - rb;
       if (it.n_iter < 0) it.n_iter = 0;
@@ -192,11 +192,19 @@ fa_bwd_kv_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     return it;
   };
   // Work list: pairs (k-th heaviest, k-th lightest key block of a slice) handed out round-robin, so that under causal
-  // masking every CTA gets the same number of blocks and neighbouring CTAs share a slice's operands in L2.
+  // masking every CTA gets the same number of blocks and neighbouring CTAs share a slice's operands in L2. SINGLES (no
+  // causal mask, chosen by fa_bwd_singles): one key block at a time.
   const int npair = (p.nrb + 1) / 2;
   const int n_super = (p.total_items / p.nrb) * npair;
-  const int n_steps = 2 * ((n_super + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x));
+  const int n_steps = SINGLES ? (p.total_items + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x)
+                              : 2 * ((n_super + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x));
   auto decode_step = [&](int u, FaBwdItem& it) -> bool {
+    if constexpr (SINGLES) {
+      const int w = u * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
+      if (w >= p.total_items) return false;
+      it = decode(w);
+      return true;
+    }
     const int sidx = (u >> 1) * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
     if (sidx >= n_super) return false;
     const int j = sidx % npair;
@@ -493,7 +501,7 @@ fa_bwd_kv_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
       }
       for (int t = 0; t < n_iter; ++t) {
         const int g = g0 + t;
-        const bool diag = p.causal && (it.t_start + t) * 128 == row0;  // the only block that straddles the diagonal
+        const bool diag = !SINGLES && p.causal && (it.t_start + t) * 128 == row0;  // the only block that straddles the diagonal
         const uint32_t tz1 = tmem_addr(tZ1, lane_base, grp * 32);
         const uint32_t tz2 = tmem_addr(tZ2, lane_base, grp * 32);
         if (threadIdx.x == 0) AB200_FBTR(0, g, 0);

@@ -31,6 +31,14 @@ struct FaBwdArgs {
   int causal;
 };
 
+// Without a causal mask all row blocks cost the same, and dealing pairs of them only makes the unit coarse: single blocks
+// where the busiest SM then holds fewer. (A specialisation rather than a choice at run time: the order evaluated at run time
+// cost the dQ kernel 5 %, B=8 H=32 L=1795 d=64 442 -> 466 us, under a causal mask.)
+inline bool fa_bwd_singles(int BH, int nrb, bool causal) {
+  const long long sms = persistent_workers(), pairs = static_cast<long long>(BH) * ((nrb + 1) / 2), items = static_cast<long long>(BH) * nrb;
+  return !causal && (items + sms - 1) / sms < 2 * ((pairs + sms - 1) / sms);
+}
+
 template <class Cfg>
 int fa_bwd_one(const void* R1, const void* R2, int r_len, const void* C1, const void* C2, const void* T, int c_len,
                FaBwdParams p, int BH, cudaStream_t stream, const char* what, bool overlap) {
@@ -42,14 +50,16 @@ int fa_bwd_one(const void* R1, const void* R2, int r_len, const void* C1, const 
   if ((rc = make_tmap_3d(&tc1, C1, Cfg::BF16, Cfg::D, c_len, BH, 64, 128))) return rc;
   if ((rc = make_tmap_3d(&tc2, C2, Cfg::BF16, Cfg::D, c_len, BH, 64, 128))) return rc;
   if ((rc = make_tmap_3d(&tt, T, Cfg::BF16, Cfg::D, c_len, BH, 64, 128))) return rc;
+  const bool singles = Cfg::WHICH == kFaBwdDQ && fa_bwd_singles(BH, (r_len + 127) / 128, p.causal != 0);
   auto kernel = &fa_bwd_sm100_kernel<Cfg>;
+  if constexpr (Cfg::WHICH == kFaBwdDQ) kernel = singles ? &fa_bwd_sm100_kernel<Cfg, true> : kernel;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
   if (e != cudaSuccess) return fail(kErrCuda, "%s: cudaFuncSetAttribute: %s", what, cudaGetErrorString(e));
   p.nrb = (r_len + 127) / 128;
   const long long total = static_cast<long long>(p.nrb) * BH;
   if (total > 0x7fffffffLL) return fail(kErrInvalidArgument, "%s: too many tiles", what);
   p.total_items = static_cast<int>(total);
-  e = launch_maybe_overlapped(kernel, persistent_grid(BH * ((p.nrb + 1) / 2)), Cfg::NTHREADS, Cfg::SMEM_BYTES, stream, overlap,
+  e = launch_maybe_overlapped(kernel, persistent_grid(singles ? p.total_items : BH * ((p.nrb + 1) / 2)), Cfg::NTHREADS, Cfg::SMEM_BYTES, stream, overlap,
                               tr1, tr2, tc1, tc2, tt, p);
   if (e != cudaSuccess) return fail(kErrCuda, "%s: %s", what, cudaGetErrorString(e));
   return check_launch(what);
@@ -72,7 +82,8 @@ int fa_bwd_kv_launch(const FaBwdArgs& a, cudaStream_t stream) {
   if ((rc = make_tmap_3d(&tv, a.v, BF16, D, a.Lkv, a.BH, 64, 128))) return rc;
   if ((rc = make_tmap_3d(&tq, a.q, BF16, D, a.Lq, a.BH, 64, 128))) return rc;
   if ((rc = make_tmap_3d(&tdo, a.dout, BF16, D, a.Lq, a.BH, 64, 128))) return rc;
-  auto kernel = &fa_bwd_kv_sm100_kernel<Cfg>;
+  const bool singles = fa_bwd_singles(a.BH, (a.Lkv + 127) / 128, a.causal != 0);
+  auto kernel = singles ? &fa_bwd_kv_sm100_kernel<Cfg, true> : &fa_bwd_kv_sm100_kernel<Cfg, false>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
   if (e != cudaSuccess) return fail(kErrCuda, "%s: cudaFuncSetAttribute: %s", what, cudaGetErrorString(e));
   FaBwdKvParams p{};
@@ -88,7 +99,7 @@ int fa_bwd_kv_launch(const FaBwdArgs& a, cudaStream_t stream) {
   const long long total = static_cast<long long>(p.nrb) * a.BH;
   if (total > 0x7fffffffLL) return fail(kErrInvalidArgument, "%s: too many tiles", what);
   p.total_items = static_cast<int>(total);
-  e = launch_maybe_overlapped(kernel, persistent_grid(a.BH * ((p.nrb + 1) / 2)), Cfg::NTHREADS, Cfg::SMEM_BYTES, stream, false,
+  e = launch_maybe_overlapped(kernel, persistent_grid(singles ? p.total_items : a.BH * ((p.nrb + 1) / 2)), Cfg::NTHREADS, Cfg::SMEM_BYTES, stream, false,
                               tk, tv, tq, tdo, p);
   if (e != cudaSuccess) return fail(kErrCuda, "%s: %s", what, cudaGetErrorString(e));
   return check_launch(what);

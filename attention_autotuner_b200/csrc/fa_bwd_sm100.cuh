@@ -163,7 +163,7 @@ __device__ __forceinline__ uint64_t fa_bwd_unpack2(uint32_t packed) {
   }
 }
 
-template <class Cfg>
+template <class Cfg, bool SINGLES = false>
 __global__ void __launch_bounds__(Cfg::NTHREADS, 1)
 fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ CUtensorMap tmR2,
                     const __grid_constant__ CUtensorMap tmC1, const __grid_constant__ CUtensorMap tmC2,
@@ -225,11 +225,11 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_const
     FaBwdItem it;
     const int k = w % p.nrb;
     it.bh = w / p.nrb;
-    const int rb = (p.causal && !ROWK) ? (p.nrb - 1 - k) : k;  // heaviest row blocks first
+    const int rb = (!SINGLES && p.causal && !ROWK) ? (p.nrb - 1 - k) : k;  // heaviest row blocks first
     it.row0 = rb * 128;
     it.t_start = 0;
     it.n_iter = ncb;
-    if (p.causal) {
+    if (!SINGLES && p.causal) {
       if (ROWK) {
         it.t_start = rb;  // query blocks before this key block see none of its keys
         it.n_iter = ncb - rb;
@@ -244,12 +244,20 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_const
   // in runs of G consecutive pairs per CTA. G = 1 keeps all CTAs on neighbouring slices (operands shared in L2); the
   // dK kernel takes G = 2, i.e. four tiles of one slice in a row, so that its helper finds three of four delta
   // tables in its cache (computing one takes about 5300 cycles, against 3200 for the rest of a block).
+  // SINGLES (dQ without a causal mask, chosen by fa_bwd_singles): one row block at a time.
   constexpr int G = (Cfg::WHICH == kFaBwdDK) ? 2 : 1;
   const int npair = (p.nrb + 1) / 2;
   const int n_super = (p.total_items / p.nrb) * npair;
   const int per_window = static_cast<int>(gridDim.x) * G;
-  const int n_steps = 2 * G * ((n_super + per_window - 1) / per_window);
+  const int n_steps = SINGLES ? (p.total_items + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x)
+                              : 2 * G * ((n_super + per_window - 1) / per_window);
   auto decode_step = [&](int u, FaBwdItem& it) -> bool {
+    if constexpr (SINGLES) {
+      const int w = u * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
+      if (w >= p.total_items) return false;
+      it = decode(w);
+      return true;
+    }
     const int s = u >> 1;
     const int sidx = ((s / G) * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x)) * G + (s % G);
     if (sidx >= n_super) return false;
@@ -507,7 +515,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_const
           }
           mbar_arrive(&tab_free[ts]);
         }
-        const bool diag = p.causal && col0 == row0;  // the only block that straddles the diagonal (Lq == Lkv)
+        const bool diag = !SINGLES && p.causal && col0 == row0;  // the only block that straddles the diagonal (Lq == Lkv)
         if (threadIdx.x == 0) AB200_FBTR(0, g, 1);
         ok = mbar_wait_warp(&z_full[g % NZ], (g / NZ) & 1, ab, kFbZFull);
         if (!ok) break;
