@@ -4,6 +4,7 @@ The knobs are Blackwell's: query tiles per CTA, depth of the TMA-fed K/V ring, V
 Feasibility = shared memory per CTA <= arch.smem_cap and tensor-memory columns <= arch.tmem_columns,
 which replace the reference's shared-memory and accumulator-register checks (tunner.py:102-151)."""
 import ctypes
+import os
 
 from .base_tunner import BaseTunner, CompileResult  # noqa: F401
 from .configs import AttnConfig, RetBwdConfig, RetConfig  # noqa: F401
@@ -21,9 +22,28 @@ def _flops_fwd(t, causal):
     return 2.0 * B * H * pairs * (dqk + dv)
 
 
+# What csrc/fa_fwd_launch.cuh (fa_fwd_is_decode) sends to the decoding kernel: up to DECODE_ROWS query rows, one head
+# dimension out of DECODE_DIMS for q, k and v, and no form of the grid asked for in the environment.
+DECODE_ROWS = 16
+DECODE_DIMS = (64, 128)
+
+
+def is_decoding(q_shape, v_shape) -> bool:
+    return (q_shape[-2] <= DECODE_ROWS and q_shape[-1] == v_shape[-1] and q_shape[-1] in DECODE_DIMS
+            and os.environ.get("ATTN_B200_FA_FWD_FORM", "")[:1] not in ("g", "p"))
+
+
 class AttnTunner(BaseTunner):
     def __init__(self, arch, torch_array: list, *, scale=None, causal=False):
         super().__init__(arch, torch_array, "attention", scale=scale, causal=causal)
+
+    def tune(self, log_path=None, *, search=None, top_k=None, force=False):
+        """As the base class, except for a decoding call: its kernel has no tile to choose and comes with the default
+        configuration. A search would time that one kernel under every name and leave the luckiest in the cache for all
+        longer calls; a cached configuration that forces a form would run the 256-row tile instead."""
+        if is_decoding(self.torch_array[0].shape, self.torch_array[2].shape):
+            return self.default_config()
+        return super().tune(log_path, search=search, top_k=top_k, force=force)
 
     def validate_kernel(self, config):
         if config.Kd % 64 != 0 or config.D % 64 != 0 or config.D % config.dv_chunk != 0:

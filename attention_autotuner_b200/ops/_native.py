@@ -17,7 +17,7 @@ import torch
 
 from .. import _lib
 from ..autotuner.runtime import KernelError, Runtime
-from ..autotuner.tunner import AttnTunner, RetBwdTunner, RetTunner
+from ..autotuner.tunner import AttnTunner, RetBwdTunner, RetTunner, is_decoding
 from ..build import OPS_PATH
 
 _ENV = ["ATTN_B200_CACHE_DIR", "ATTN_B200_AUTOTUNE"]
@@ -53,13 +53,16 @@ def ops():
     return _module
 
 
+def _make_plan(tuner, cfg, files, env):
+    rt = Runtime(tuner.arch, cfg)
+    lib = rt._lib()
+    return ops().make_plan(_address(lib.kernel_entry_ex), _address(lib.last_error), rt.libname, files, env)
+
+
 def _resolve(tuner, key):
     """Plan of the configuration the tuner picks. Remembered unless the pick was neither read from the tuning cache nor
     the built-in tile by request (then the tuner is asked again next time, as a failed search should be)."""
-    cfg = tuner.tune()
-    rt = Runtime(tuner.arch, cfg)
-    lib = rt._lib()
-    plan = ops().make_plan(_address(lib.kernel_entry_ex), _address(lib.last_error), rt.libname, tuner.cache_candidates(), _ENV)
+    plan = _make_plan(tuner, tuner.tune(), tuner.cache_candidates(), _ENV)
     if tuner.check_cache() is not None or os.environ.get("ATTN_B200_AUTOTUNE", "1") == "0":
         _plans[key] = plan
     return plan
@@ -69,15 +72,24 @@ def _key(op, arch, dqk, dv, dtype, flag):
     return (op, type(arch), arch.compute_capability, dqk, dv, dtype, flag)
 
 
+def _attn_key(arch, q, v, causal):
+    op = "attn_decode" if is_decoding(q.shape, v.shape) else "attn"
+    return _key(op, arch, q.shape[-1], v.shape[-1], q.dtype, bool(causal))
+
+
 def attn_plan(arch, q, v, causal):
-    return _plans.get(_key("attn", arch, q.shape[-1], v.shape[-1], q.dtype, bool(causal)))
+    return _plans.get(_attn_key(arch, q, v, causal))
 
 
 def resolve_attn(arch, q, k, v, causal, scale):
     o = torch.empty(*q.shape[:3], v.shape[3], device=q.device, dtype=q.dtype)  # a search times the kernels on these tensors
     tuner = AttnTunner(arch=arch, torch_array=[q.detach().contiguous(), k.detach().contiguous(), v.detach().contiguous(), o],
                        scale=scale, causal=causal)
-    return _resolve(tuner, _key("attn", arch, q.shape[-1], v.shape[-1], q.dtype, bool(causal)))
+    if is_decoding(q.shape, v.shape):
+        plan = _make_plan(tuner, tuner.tune(), [], ["ATTN_B200_FA_FWD_FORM"])  # the cache has no part in it
+        _plans[_attn_key(arch, q, v, causal)] = plan
+        return plan
+    return _resolve(tuner, _attn_key(arch, q, v, causal))
 
 
 def _ret_flag(causal, has_decay):

@@ -1,0 +1,96 @@
+"""Which configuration serves a decoding call (up to 16 query rows, csrc/fa_decode_sm100.cuh), without a GPU: the default
+one, neither searched for nor read from or written to the tuning cache, and kept apart from that of longer calls."""
+import json
+import os
+import re
+
+import pytest
+import torch
+
+from attention_autotuner_b200.arch import B200
+from attention_autotuner_b200.autotuner import tunner
+from attention_autotuner_b200.autotuner.configs import AttnConfig
+from attention_autotuner_b200.autotuner.tunner import AttnTunner
+from attention_autotuner_b200.build import CSRC
+
+
+def tensors(Lq, d, dv=None, dt=torch.bfloat16):
+    q, k = torch.zeros(1, 2, Lq, d, dtype=dt), torch.zeros(1, 2, 64, d, dtype=dt)
+    return [q, k, torch.zeros(1, 2, 64, dv or d, dtype=dt), torch.zeros(1, 2, Lq, dv or d, dtype=dt)]
+
+
+class Searched(Exception):
+    pass
+
+
+@pytest.fixture
+def searching(monkeypatch, tmp_path):
+    """Searches enabled, as with a GPU; one that starts raises Searched. Returns the cache's folder."""
+    def start(*_a, **_k):
+        raise Searched
+    monkeypatch.setenv("ATTN_B200_CACHE_DIR", str(tmp_path))
+    monkeypatch.setenv("ATTN_B200_AUTOTUNE", "1")
+    monkeypatch.delenv("ATTN_B200_FA_FWD_FORM", raising=False)
+    monkeypatch.setattr(torch.cuda, "is_available", lambda: True)
+    monkeypatch.setattr(AttnTunner, "compile_parallel", start)
+    return tmp_path
+
+
+@pytest.mark.parametrize("Lq,d", [(1, 64), (1, 128), (16, 64), (16, 128)])
+def test_a_decoding_call_neither_searches_nor_stores(searching, monkeypatch, Lq, d):
+    t = AttnTunner(B200(), tensors(Lq, d), causal=True)
+    assert t.tune() == t.default_config() and t.tune(force=True) == t.default_config()
+    assert os.listdir(searching) == []
+    # a cached configuration that forces a form of the grid does not keep it from the decoding kernel
+    cached = AttnConfig(256, 128, d, d, q_tiles=2, kv_stages=4, dv_chunk=d, persistent=1, dtype="bf16")
+    with open(t._cache_file(), "w") as f:
+        json.dump(cached.to_dict(), f)
+    assert t.tune() == t.default_config() and t.default_config().substitution_map()["launcher"] == "fa_fwd_launch_auto"
+    # calls the large tiles serve: one row more, other head dimensions, a form asked for
+    assert AttnTunner(B200(), tensors(17, d), causal=True).tune() == cached
+    with pytest.raises(Searched):
+        AttnTunner(B200(), tensors(Lq, d, 192), causal=True).tune()
+    monkeypatch.setenv("ATTN_B200_FA_FWD_FORM", "grid")
+    assert AttnTunner(B200(), tensors(Lq, d), causal=True).tune() == cached
+
+
+def test_the_plan_of_a_decoding_call_is_its_own(searching, monkeypatch):
+    from attention_autotuner_b200.ops import _native
+
+    class Library:  # stands in for the per-configuration library: which one is asked for is what the test looks at
+        def __init__(self, arch, config):
+            self.libname = str(config)
+            asked.append(config)
+
+        def _lib(self):
+            class L:
+                kernel_entry_ex = last_error = None
+            return L
+
+    asked = []
+    monkeypatch.setattr(_native, "Runtime", Library)
+    monkeypatch.setattr(_native, "_address", lambda fn: 0)
+    monkeypatch.setattr(_native, "_plans", {})
+    arch = B200()
+    one, many = tensors(1, 128), tensors(17, 128)
+    cached = AttnConfig(256, 128, 128, 128, q_tiles=2, kv_stages=3, dv_chunk=128, cta_pair=1, dtype="bf16")
+    plan = _native.resolve_attn(arch, *one[:3], True, 1.0)
+    assert asked[-1] == AttnTunner(arch, one).default_config() and _native.attn_plan(arch, one[0], one[2], True) is plan
+    assert _native.attn_plan(arch, many[0], many[2], True) is None
+    with open(AttnTunner(arch, many, causal=True)._cache_file(), "w") as f:
+        json.dump(cached.to_dict(), f)
+    assert _native.resolve_attn(arch, *many[:3], True, 1.0) is _native.attn_plan(arch, many[0], many[2], True)
+    assert asked[-1] == cached and _native.ops().plan_fresh(plan)
+    # a form asked for in the environment ends the decoding plan
+    monkeypatch.setenv("ATTN_B200_FA_FWD_FORM", "persistent")
+    assert not _native.ops().plan_fresh(plan) and _native.attn_plan(arch, one[0], one[2], True) is not plan
+
+
+def test_the_rule_is_the_launchers():
+    with open(os.path.join(CSRC, "fa_decode_sm100.cuh")) as f:
+        rows = re.search(r"int MAX_ROWS = (\d+);", f.read())
+    with open(os.path.join(CSRC, "fa_fwd_launch.cuh")) as f:
+        rule = re.search(r"bool fa_fwd_is_decode\(.*?\n}", f.read(), re.S).group(0)
+    assert int(rows.group(1)) == tunner.DECODE_ROWS
+    assert [int(x) for x in re.findall(r"Cfg::DQK == (\d+)", rule)] == list(tunner.DECODE_DIMS)
+    assert re.findall(r"a\.Lq <= (\d+)", rule) == [str(tunner.DECODE_ROWS)] and "a.dv == Cfg::DQK" in rule
