@@ -1,8 +1,8 @@
 """The native operator layer (csrc/host/torch_ops.cpp, built into _torch_ops.so) and the plans it is called with.
 
 A plan names the per-configuration library entry point that serves a call. It is resolved by the tuner exactly as before
-(tuning-cache file, search, or the built-in tile) and remembered per (operation, head dimensions, dtype, mask form)
-together with everything the choice was read from: the cache files' modification times and the environment variables.
+(tuning-cache file, search, or the built-in tile) and remembered per (operation, device limits, head dimensions, dtype,
+mask form) together with everything the choice was read from: the cache files' modification times and the environment variables.
 The native layer compares those on every call (two ``stat`` calls) and refuses a stale plan, so a cache entry written
 by this or another process takes effect at the next call, as it did when the tuner ran on every call."""
 from __future__ import annotations
@@ -69,7 +69,9 @@ def _resolve(tuner, key):
 
 
 def _key(op, arch, dqk, dv, dtype, flag):
-    return (op, type(arch), arch.compute_capability, dqk, dv, dtype, flag)
+    # of the device description: what names the cache file and the library, and the limits that bound the tiles
+    return (op, type(arch), getattr(arch, "compute_capability", ""), getattr(arch, "smem_cap", None),
+            getattr(arch, "tmem_columns", None), dqk, dv, dtype, flag)
 
 
 def _attn_key(arch, q, v, causal):

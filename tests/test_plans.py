@@ -1,5 +1,6 @@
-"""Which configuration serves a decoding call (up to 16 query rows, csrc/fa_decode_sm100.cuh), without a GPU: the default
-one, neither searched for nor read from or written to the tuning cache, and kept apart from that of longer calls."""
+"""Which configuration, and which plan of the native operator layer, serves a call; without a GPU. A decoding call (up to 16
+query rows, csrc/fa_decode_sm100.cuh) takes the default one, neither searched for nor read from or written to the tuning
+cache, and kept apart from that of longer calls."""
 import json
 import os
 import re
@@ -36,6 +37,29 @@ def searching(monkeypatch, tmp_path):
     return tmp_path
 
 
+@pytest.fixture
+def asked(monkeypatch):
+    """Plans without libraries: the configurations whose library was asked for, in order."""
+    from attention_autotuner_b200.ops import _native
+    configs = []
+
+    class Library:
+        def __init__(self, arch, config):
+            self.libname = str(config)
+            configs.append(config)
+
+        def _lib(self):
+            class L:
+                kernel_entry_ex = last_error = None
+            return L
+
+    _native.ops()
+    monkeypatch.setattr(_native, "Runtime", Library)
+    monkeypatch.setattr(_native, "_address", lambda fn: 0)
+    monkeypatch.setattr(_native, "_plans", {})
+    return configs
+
+
 @pytest.mark.parametrize("Lq,d", [(1, 64), (1, 128), (16, 64), (16, 128)])
 def test_a_decoding_call_neither_searches_nor_stores(searching, monkeypatch, Lq, d):
     t = AttnTunner(B200(), tensors(Lq, d), causal=True)
@@ -54,23 +78,8 @@ def test_a_decoding_call_neither_searches_nor_stores(searching, monkeypatch, Lq,
     assert AttnTunner(B200(), tensors(Lq, d), causal=True).tune() == cached
 
 
-def test_the_plan_of_a_decoding_call_is_its_own(searching, monkeypatch):
+def test_the_plan_of_a_decoding_call_is_its_own(searching, asked, monkeypatch):
     from attention_autotuner_b200.ops import _native
-
-    class Library:  # stands in for the per-configuration library: which one is asked for is what the test looks at
-        def __init__(self, arch, config):
-            self.libname = str(config)
-            asked.append(config)
-
-        def _lib(self):
-            class L:
-                kernel_entry_ex = last_error = None
-            return L
-
-    asked = []
-    monkeypatch.setattr(_native, "Runtime", Library)
-    monkeypatch.setattr(_native, "_address", lambda fn: 0)
-    monkeypatch.setattr(_native, "_plans", {})
     arch = B200()
     one, many = tensors(1, 128), tensors(17, 128)
     cached = AttnConfig(256, 128, 128, 128, q_tiles=2, kv_stages=3, dv_chunk=128, cta_pair=1, dtype="bf16")
@@ -84,6 +93,24 @@ def test_the_plan_of_a_decoding_call_is_its_own(searching, monkeypatch):
     # a form asked for in the environment ends the decoding plan
     monkeypatch.setenv("ATTN_B200_FA_FWD_FORM", "persistent")
     assert not _native.ops().plan_fresh(plan) and _native.attn_plan(arch, one[0], one[2], True) is not plan
+
+
+def test_device_descriptions_with_other_limits_have_plans_of_their_own(asked, monkeypatch, tmp_path):
+    from attention_autotuner_b200.ops import _native
+    monkeypatch.setenv("ATTN_B200_CACHE_DIR", str(tmp_path))
+    monkeypatch.setenv("ATTN_B200_AUTOTUNE", "0")
+    q, k, v, _o = tensors(256, 128)
+    wide, small, few = B200(), B200(), B200()
+    small.smem_cap = 160 * 1024  # a K / V ring of two entries beside two query tiles, or one query tile
+    few.tmem_columns = 256       # no room for two query tiles
+    plans = []
+    for arch in (wide, small, few):
+        assert _native.attn_plan(arch, q, v, True) is None
+        plans.append(_native.resolve_attn(arch, q, k, v, True, 1.0))
+        assert AttnTunner(arch, [q, k, v, v]).validate_kernel(asked[-1])
+    assert len({str(c) for c in asked}) == 3
+    assert [_native.attn_plan(a, q, v, True) for a in (wide, small, few)] == plans
+    assert _native.attn_plan(B200(), q, v, True) is plans[0]
 
 
 def test_the_rule_is_the_launchers():
