@@ -44,6 +44,10 @@ def _dtype_name(t: torch.Tensor) -> str:
     return "bf16" if t.dtype == torch.bfloat16 else "fp16"
 
 
+def cache_dir() -> str:
+    return os.environ.get("ATTN_B200_CACHE_DIR", os.path.join(PKG_DIR, "cache"))
+
+
 _CACHE_MEMO: dict = {}  # cache file path -> (mtime_ns, parsed configuration or None)
 
 
@@ -55,7 +59,7 @@ class BaseTunner:
         self.Br_list = [128, 256]
         self.Bc_list = [128]
         self.op_name = op_name
-        self.cache_path = os.environ.get("ATTN_B200_CACHE_DIR", os.path.join(PKG_DIR, "cache"))
+        self.cache_path = cache_dir()
         self.problem_key = {
             "dim_qk": torch_array[0].shape[-1],
             "dim_v": torch_array[2].shape[-1],

@@ -69,6 +69,7 @@ struct Plan {
   };
   std::vector<Env> env;
 
+  bool usable() const { return fn != nullptr && fresh(); }
   bool fresh() const {
     for (const auto& e : env) {
       const char* now = getenv(e.name.c_str());
@@ -248,7 +249,7 @@ variable_list ret_backward(const Tensor& q, const Tensor& k, const Tensor& v, co
   c10::cuda::CUDAGuard guard(q.device());
   Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);
   Tensor scratch = ret_bwd_scratch(q, k, mask);
-  if (plan == nullptr || !plan->fresh()) {
+  if (plan == nullptr || !plan->usable()) {
     // not looked up yet (or changed since): the Python side resolves it, with these tensors should it want to search
     py::gil_scoped_acquire gil;
     auto wrap = [](const Tensor& t) { return py::reinterpret_steal<py::object>(THPVariable_Wrap(t)); };
@@ -342,7 +343,7 @@ PyObject* py_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Tensor o, lse;
   {
     py::gil_scoped_release nogil;
-    if (!plan->fresh()) plan = nullptr;
+    if (!plan->usable()) plan = nullptr;
     else if (any_grad(q, k, v)) {
       variable_list out = AttnNode::apply(q, k, v, reinterpret_cast<int64_t>(plan), scale, causal != 0, ret_lse != 0);
       o = out[0];
@@ -379,7 +380,7 @@ PyObject* py_retnet(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Tensor o;
   {
     py::gil_scoped_release nogil;
-    if (!plan->fresh()) plan = nullptr;
+    if (!plan->usable()) plan = nullptr;
     else if (any_grad(q, k, v)) {
       auto given = [](const Tensor& t) { return t.defined() ? std::optional<Tensor>(t) : std::nullopt; };
       o = RetNode::apply(q, k, v, given(mask), given(decay), reinterpret_cast<int64_t>(plan), reinterpret_cast<int64_t>(bwd),
@@ -413,7 +414,7 @@ PyObject* py_retnet_fwd_raw(PyObject*, PyObject* const* a, Py_ssize_t n) {
   {
     py::gil_scoped_release nogil;
     at::NoGradGuard no_grad;
-    if (!plan->fresh()) plan = nullptr;
+    if (!plan->usable()) plan = nullptr;
     else {
       if (mask.defined()) m = mask.detach().contiguous();
       d = decay_on(decay, q);
@@ -487,7 +488,10 @@ PyObject* py_chunkwise(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// make_plan(entry point, last_error, library name, [paths], [environment variables]) -> plan
+// make_plan(entry point, last_error, library name, [paths], [environment variables]) -> plan, stamped with the files' times
+// and the variables' values of this moment. What the plan is made from is to be read after that: then a change in between
+// makes the plan stale instead of being taken as seen. The entry point may follow with set_entry; a plan without one is
+// declined by every function.
 PyObject* py_make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (!arg_count(n, 5, "make_plan")) return nullptr;
@@ -505,6 +509,19 @@ PyObject* py_make_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
     plan->env.push_back({name, now ? now : "", now != nullptr});
   }
   return PyCapsule_New(plan, kPlanName, nullptr);
+  END_HANDLE_TH_ERRORS
+}
+
+// set_entry(plan, entry point, last_error, library name); before the plan is handed to any other function
+PyObject* py_set_entry(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  if (!arg_count(n, 4, "set_entry")) return nullptr;
+  Plan* plan = take_plan(a[0]);
+  if (plan == nullptr) return PyErr_Occurred() ? nullptr : none();
+  plan->last_error = reinterpret_cast<LastErrorFn>(py::cast<uintptr_t>(py::handle(a[2])));
+  plan->libname = py::cast<std::string>(py::handle(a[3]));
+  plan->fn = reinterpret_cast<void*>(py::cast<uintptr_t>(py::handle(a[1])));
+  Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }
 
@@ -544,6 +561,7 @@ PyMethodDef g_methods[] = {
     {"retnet_bwd_raw", fast(py_retnet_bwd_raw), METH_FASTCALL, nullptr},
     {"chunkwise", fast(py_chunkwise), METH_FASTCALL, nullptr},
     {"make_plan", fast(py_make_plan), METH_FASTCALL, nullptr},
+    {"set_entry", fast(py_set_entry), METH_FASTCALL, nullptr},
     {"plan_fresh", py_plan_fresh, METH_O, nullptr},
     {"init", fast(py_init), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};

@@ -16,11 +16,13 @@ import threading
 import torch
 
 from .. import _lib
+from ..autotuner.base_tunner import cache_dir
 from ..autotuner.runtime import KernelError, Runtime
 from ..autotuner.tunner import AttnTunner, RetBwdTunner, RetTunner, is_decoding
 from ..build import OPS_PATH
 
 _ENV = ["ATTN_B200_CACHE_DIR", "ATTN_B200_AUTOTUNE"]
+TRIES = 16  # attempts at a call that no change of the tuning cache overtakes; each change costs one
 
 _lock = threading.Lock()
 _module = None
@@ -53,19 +55,32 @@ def ops():
     return _module
 
 
-def _make_plan(tuner, cfg, files, env):
+def _set_entry(plan, tuner, cfg):
     rt = Runtime(tuner.arch, cfg)
     lib = rt._lib()
-    return ops().make_plan(_address(lib.kernel_entry_ex), _address(lib.last_error), rt.libname, files, env)
+    ops().set_entry(plan, _address(lib.kernel_entry_ex), _address(lib.last_error), rt.libname)
+    return plan
 
 
 def _resolve(tuner, key):
     """Plan of the configuration the tuner picks. Remembered unless the pick was neither read from the tuning cache nor
-    the built-in tile by request (then the tuner is asked again next time, as a failed search should be)."""
-    plan = _make_plan(tuner, tuner.tune(), tuner.cache_candidates(), _ENV)
-    if tuner.check_cache() is not None or os.environ.get("ATTN_B200_AUTOTUNE", "1") == "0":
-        _plans[key] = plan
-    return plan
+    the built-in tile by request (then the tuner is asked again next time, as a failed search should be).
+
+    The plan is stamped before the cache is read, and the choice is made again if an entry was written in the meantime
+    (by the search itself, or by another process while this one was compiling the library)."""
+    native = ops()
+    for _ in range(TRIES):
+        plan = native.make_plan(0, 0, "", tuner.cache_candidates(), _ENV)
+        if tuner.cache_path != cache_dir():  # another folder since the tuner was made
+            tuner.cache_path = cache_dir()
+            continue
+        cached = tuner.check_cache()
+        _set_entry(plan, tuner, tuner.tune() if cached is None else cached)
+        if native.plan_fresh(plan):
+            if cached is not None or os.environ.get("ATTN_B200_AUTOTUNE", "1") == "0":
+                _plans[key] = plan
+            return plan
+    raise RuntimeError("the tuning cache keeps changing while a call is being prepared")
 
 
 def _key(op, arch, dqk, dv, dtype, flag):
@@ -88,7 +103,7 @@ def resolve_attn(arch, q, k, v, causal, scale):
     tuner = AttnTunner(arch=arch, torch_array=[q.detach().contiguous(), k.detach().contiguous(), v.detach().contiguous(), o],
                        scale=scale, causal=causal)
     if is_decoding(q.shape, v.shape):
-        plan = _make_plan(tuner, tuner.tune(), [], ["ATTN_B200_FA_FWD_FORM"])  # the cache has no part in it
+        plan = _set_entry(ops().make_plan(0, 0, "", [], ["ATTN_B200_FA_FWD_FORM"]), tuner, tuner.tune())  # no cache entry in it
         _plans[_attn_key(arch, q, v, causal)] = plan
         return plan
     return _resolve(tuner, _attn_key(arch, q, v, causal))

@@ -10,7 +10,7 @@ flash-attention backward kernels (csrc/fa_bwd_kv_sm100.cuh, csrc/fa_bwd_sm100.cu
 raises for every other shape instead of returning None.
 """
 from ._checks import check_qkv
-from ._native import attn_plan, ops, resolve_attn
+from ._native import TRIES, attn_plan, ops, resolve_attn
 
 
 def flash_attn_func(q, k, v, device_type, causal=False, softmax_scale=None, return_lse=False):
@@ -21,13 +21,15 @@ def flash_attn_func(q, k, v, device_type, causal=False, softmax_scale=None, retu
     except (AttributeError, IndexError):
         plan = None  # not tensors: the checks below say so
     out = native.attn(q, k, v, plan, scale, causal, return_lse) if plan is not None else None
-    if out is None:
+    for _ in range(TRIES):
+        if out is not None:
+            return out
         # first call for these head dimensions, a changed tuning cache, or arguments the kernels do not take (raises)
         check_qkv("flash_attn_func", q, k, v)
         plan = resolve_attn(device_type, q, k, v, causal, softmax_scale)
         out = native.attn(q, k, v, plan, scale, causal, return_lse)
-        if out is None:
-            raise RuntimeError("flash_attn_func: the tuning cache changed while the call was being prepared")
+    if out is None:
+        raise RuntimeError("flash_attn_func: the tuning cache keeps changing while the call is being prepared")
     return out
 
 

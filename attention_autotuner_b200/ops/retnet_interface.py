@@ -11,7 +11,7 @@ tensor, ``causal=True`` declares it lower triangular so the kernels skip the blo
 import torch
 
 from ._checks import check_like, check_mask_decay, check_qkv
-from ._native import arch_token, ops, resolve_ret, ret_plan
+from ._native import TRIES, arch_token, ops, resolve_ret, ret_plan
 
 
 def _plan_or_none(op, arch, q, v, causal, decay):
@@ -25,12 +25,14 @@ def _call(native_call, device_type, q, k, v, mask, causal, scale, decay):
     """native_call(plan), with the checks and the plan's resolution where the first try declines."""
     plan = _plan_or_none("ret", device_type, q, v, causal, decay)
     out = native_call(plan) if plan is not None else None
-    if out is None:
+    for _ in range(TRIES):
+        if out is not None:
+            return out
         check_qkv("RetNetAttnFunc", q, k, v)
         check_mask_decay("RetNetAttnFunc", q, k, mask, decay)
         out = native_call(resolve_ret(device_type, q, k, v, mask, causal, scale, decay))
-        if out is None:
-            raise RuntimeError("RetNetAttnFunc: the tuning cache changed while the call was being prepared")
+    if out is None:
+        raise RuntimeError("RetNetAttnFunc: the tuning cache keeps changing while the call is being prepared")
     return out
 
 

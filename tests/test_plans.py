@@ -113,6 +113,55 @@ def test_device_descriptions_with_other_limits_have_plans_of_their_own(asked, mo
     assert _native.attn_plan(B200(), q, v, True) is plans[0]
 
 
+def test_an_entry_written_while_a_plan_is_made_is_not_taken_as_seen(asked, monkeypatch, tmp_path):
+    """Another process stores an entry while this one compiles the library of the choice it has read before."""
+    from attention_autotuner_b200.ops import _native
+    monkeypatch.setenv("ATTN_B200_CACHE_DIR", str(tmp_path))
+    monkeypatch.setenv("ATTN_B200_AUTOTUNE", "0")
+    arch, (q, k, v, o) = B200(), tensors(256, 128)
+    path = AttnTunner(arch, [q, k, v, o], causal=True)._cache_file()
+    entries = [AttnConfig(256, 128, 128, 128, q_tiles=2, kv_stages=s, dv_chunk=128, persistent=p, dtype="bf16") for s, p in ((3, 0), (3, 1))]
+    left = list(entries)
+    library = _native.Runtime
+
+    def slow(arch, config):
+        if left:
+            with open(path, "w") as f:
+                json.dump(left[0].to_dict(), f)
+            os.utime(path, ns=(len(left), len(left)))
+            left.pop(0)
+        return library(arch, config)
+
+    monkeypatch.setattr(_native, "Runtime", slow)
+    plan = _native.resolve_attn(arch, q, k, v, True, 1.0)
+    assert asked == [AttnTunner(arch, [q, k, v, o]).default_config(), *entries]
+    assert _native.attn_plan(arch, q, v, True) is plan and _native.ops().plan_fresh(plan)
+
+
+def test_an_operator_prepares_again_what_a_change_has_overtaken(monkeypatch):
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from attention_autotuner_b200.ops import attention_interface, retnet_interface
+    with FakeTensorMode():
+        q = torch.empty(1, 2, 64, 128, dtype=torch.float16, device="cuda")
+    for declined in (2, 1000):
+        class Native:
+            attn = retnet = staticmethod(lambda *a: next(answers))
+
+        for mod, resolve in ((attention_interface, "resolve_attn"), (retnet_interface, "resolve_ret")):
+            monkeypatch.setattr(mod, "ops", lambda: Native)
+            monkeypatch.setattr(mod, resolve, lambda *a: "plan")
+        calls = (lambda: attention_interface.flash_attn_func(q, q, q, B200()),
+                 lambda: retnet_interface.RetNetAttnFunc(q, q, q, None, B200(), decay=torch.ones(2)))
+        for call in calls:
+            answers = iter([None] * declined + ["out"])
+            if declined == 2:
+                assert call() == "out"
+            else:
+                with pytest.raises(RuntimeError, match="keeps changing"):
+                    call()
+
+
 def test_the_rule_is_the_launchers():
     with open(os.path.join(CSRC, "fa_decode_sm100.cuh")) as f:
         rows = re.search(r"int MAX_ROWS = (\d+);", f.read())
