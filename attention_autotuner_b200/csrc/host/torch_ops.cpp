@@ -69,17 +69,25 @@ struct Plan {
   };
   std::vector<Env> env;
 
-  bool usable() const { return fn != nullptr && fresh(); }
-  bool fresh() const {
+  // The GIL is held: assignments to os.environ call setenv under it, and getenv beside a setenv is undefined.
+  bool env_unchanged() const {
+    TORCH_INTERNAL_ASSERT(PyGILState_Check(), "a plan's environment is read without the GIL");
     for (const auto& e : env) {
       const char* now = getenv(e.name.c_str());
       if ((now != nullptr) != e.set || (now != nullptr && e.value != now)) return false;
     }
+    return true;
+  }
+  // file-system calls: without the GIL where a call may
+  bool files_unchanged() const {
     for (const auto& f : files)
       if (mtime_ns(f.first) != f.second) return false;
     return true;
   }
 };
+
+// The part of a plan's check that needs the GIL; its files are looked at after the GIL is released.
+bool callable_now(const Plan* plan) { return plan->fn != nullptr && plan->env_unchanged(); }
 
 constexpr const char* kPlanName = "attn_b200.plan";
 
@@ -249,7 +257,15 @@ variable_list ret_backward(const Tensor& q, const Tensor& k, const Tensor& v, co
   c10::cuda::CUDAGuard guard(q.device());
   Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);
   Tensor scratch = ret_bwd_scratch(q, k, mask);
-  if (plan == nullptr || !plan->usable()) {
+  if (plan != nullptr) {
+    bool current = plan->files_unchanged();
+    if (current) {
+      py::gil_scoped_acquire gil;
+      current = callable_now(plan);
+    }
+    if (!current) plan = nullptr;
+  }
+  if (plan == nullptr) {
     // not looked up yet (or changed since): the Python side resolves it, with these tensors should it want to search
     py::gil_scoped_acquire gil;
     auto wrap = [](const Tensor& t) { return py::reinterpret_steal<py::object>(THPVariable_Wrap(t)); };
@@ -336,6 +352,7 @@ PyObject* py_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!take_tensor(a[0], q) || !take_tensor(a[1], k) || !take_tensor(a[2], v) || !qkv_ok(q, k, v)) return none();
   Plan* plan = take_plan(a[3]);
   if (plan == nullptr) return PyErr_Occurred() ? nullptr : none();
+  if (!callable_now(plan)) return none();
   const double scale = PyFloat_AsDouble(a[4]);
   if (scale == -1.0 && PyErr_Occurred()) return nullptr;
   const int causal = PyObject_IsTrue(a[5]), ret_lse = PyObject_IsTrue(a[6]);
@@ -343,7 +360,7 @@ PyObject* py_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Tensor o, lse;
   {
     py::gil_scoped_release nogil;
-    if (!plan->usable()) plan = nullptr;
+    if (!plan->files_unchanged()) plan = nullptr;
     else if (any_grad(q, k, v)) {
       variable_list out = AttnNode::apply(q, k, v, reinterpret_cast<int64_t>(plan), scale, causal != 0, ret_lse != 0);
       o = out[0];
@@ -371,7 +388,7 @@ PyObject* py_retnet(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Plan* plan = take_plan(a[5]);
   Plan* bwd = take_plan(a[6]);
   if (PyErr_Occurred()) return nullptr;
-  if (plan == nullptr) return none();
+  if (plan == nullptr || !callable_now(plan)) return none();
   const long long token = PyLong_AsLongLong(a[7]);
   const double scale = PyFloat_AsDouble(a[8]);
   if (PyErr_Occurred()) return nullptr;
@@ -380,7 +397,7 @@ PyObject* py_retnet(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Tensor o;
   {
     py::gil_scoped_release nogil;
-    if (!plan->usable()) plan = nullptr;
+    if (!plan->files_unchanged()) plan = nullptr;
     else if (any_grad(q, k, v)) {
       auto given = [](const Tensor& t) { return t.defined() ? std::optional<Tensor>(t) : std::nullopt; };
       o = RetNode::apply(q, k, v, given(mask), given(decay), reinterpret_cast<int64_t>(plan), reinterpret_cast<int64_t>(bwd),
@@ -406,6 +423,7 @@ PyObject* py_retnet_fwd_raw(PyObject*, PyObject* const* a, Py_ssize_t n) {
     return none();
   Plan* plan = take_plan(a[5]);
   if (plan == nullptr) return PyErr_Occurred() ? nullptr : none();
+  if (!callable_now(plan)) return none();
   const double scale = PyFloat_AsDouble(a[6]);
   if (scale == -1.0 && PyErr_Occurred()) return nullptr;
   const int causal = PyObject_IsTrue(a[7]);
@@ -414,7 +432,7 @@ PyObject* py_retnet_fwd_raw(PyObject*, PyObject* const* a, Py_ssize_t n) {
   {
     py::gil_scoped_release nogil;
     at::NoGradGuard no_grad;
-    if (!plan->usable()) plan = nullptr;
+    if (!plan->files_unchanged()) plan = nullptr;
     else {
       if (mask.defined()) m = mask.detach().contiguous();
       d = decay_on(decay, q);
@@ -528,7 +546,7 @@ PyObject* py_set_entry(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* py_plan_fresh(PyObject*, PyObject* obj) {
   Plan* plan = take_plan(obj);
   if (plan == nullptr && PyErr_Occurred()) return nullptr;
-  return PyBool_FromLong(plan != nullptr && plan->fresh());
+  return PyBool_FromLong(plan != nullptr && plan->env_unchanged() && plan->files_unchanged());
 }
 
 // init(KernelError, AttnB200Error, resolver of backward plans, last_error, fa_bwd, chunk workspace bytes, chunk forward)

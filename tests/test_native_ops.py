@@ -26,6 +26,50 @@ def test_plan_goes_stale_with_its_files_and_environment(tmp_path, monkeypatch):
     assert not native.plan_fresh(None)
 
 
+def test_a_plan_reads_the_environment_under_the_gil(monkeypatch):
+    """os.environ assignments of other threads run setenv under the GIL, so getenv has to as well. A plan with many variables,
+    the last one changed: no other thread gets to run while the call looks at them and declines."""
+    import sys
+    import threading
+    import time
+
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    from attention_autotuner_b200.ops import _native
+    native = _native.ops()
+    with FakeTensorMode():  # passes the checks of a CUDA tensor; a declined call launches nothing
+        q = torch.empty(1, 2, 64, 64, dtype=torch.float16, device="cuda")
+    decay = torch.ones(2)
+    names = [f"ATTN_B200_X{i}" for i in range(100000)]
+    plan = native.make_plan(1, 1, "lib", [], names)
+    monkeypatch.setenv(names[-1], "1")
+    turns, stop = [0], threading.Event()
+
+    def other():
+        while not stop.is_set():
+            turns[0] += 1
+            time.sleep(0)
+
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1000.0)  # a thread gives the GIL away on its own or not at all
+    thread = threading.Thread(target=other)
+    thread.start()
+    try:
+        time.sleep(0.05)
+        for call in (lambda: native.attn(q, q, q, plan, 1.0, False, False),
+                     lambda: native.retnet(q, q, q, None, decay, plan, None, 0, 1.0, True),
+                     lambda: native.retnet_fwd_raw(q, q, q, None, decay, plan, 1.0, True), lambda: native.plan_fresh(plan) or None):
+            time.sleep(0.01)
+            before = turns[0]
+            out = call()
+            after = turns[0]
+            assert out is None and before > 0 and after == before
+    finally:
+        stop.set()
+        sys.setswitchinterval(interval)
+        thread.join()
+
+
 def test_declines_what_the_python_checks_word():
     from attention_autotuner_b200.arch import B200
     from attention_autotuner_b200.ops import _native
