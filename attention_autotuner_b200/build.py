@@ -81,17 +81,24 @@ OPS_SRC = os.path.join(CSRC, "host", "torch_ops.cpp")
 OPS_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_torch_ops.so")
 
 
+OPS_FLAGS = ["-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden"]
+OPS_LIBS = ["-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+
+
 def _ops_hash() -> str:
+    """What the extension is made from: its source, the C ABI it calls, the flags, and the PyTorch and Python it is for."""
     import hashlib
     import torch
-    h = hashlib.sha1(f"{torch.__version__} {sys.version_info[:2]}".encode())
-    with open(OPS_SRC, "rb") as f:
-        h.update(f.read())
+    h = hashlib.sha1(f"{torch.__version__} {sys.version_info[:2]} {OPS_FLAGS} {OPS_LIBS}".encode())
+    for path in (OPS_SRC, os.path.join(CSRC, "..", "..", "include", "attn_b200.h")):
+        with open(path, "rb") as f:
+            h.update(f.read())
     return h.hexdigest()
 
 
 def build_torch_ops(force: bool = False) -> str:
-    """Compiles csrc/host/torch_ops.cpp into _torch_ops.so; rebuilt when the source or the PyTorch version changes."""
+    """Compiles csrc/host/torch_ops.cpp into _torch_ops.so; rebuilt when anything in _ops_hash changes. The extension carries
+    that hash, and ops/_native.py refuses to load one that was made from something else."""
     stamp = OPS_PATH + ".srchash"
     want = _ops_hash()
     try:
@@ -107,9 +114,8 @@ def build_torch_ops(force: bool = False) -> str:
     torch_dir = os.path.dirname(torch.__file__)
     incs = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
             os.path.join(cuda_home, "include"), sysconfig.get_paths()["include"]]
-    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{d}" for d in incs], OPS_SRC, "-o", OPS_PATH,
-           f"-L{os.path.join(torch_dir, 'lib')}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+    cmd = ["g++", *OPS_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DATTN_B200_OPS_HASH="{want}"',
+           *[f"-I{d}" for d in incs], OPS_SRC, "-o", OPS_PATH, f"-L{os.path.join(torch_dir, 'lib')}", *OPS_LIBS]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)

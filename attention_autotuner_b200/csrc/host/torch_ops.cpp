@@ -588,4 +588,9 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_torch_ops", nullptr, -1, g_meth
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__torch_ops() { return PyModule_Create(&g_module); }
+// build.py passes the hash of what the module is made from; ops/_native.py compares it when it loads the module
+PyMODINIT_FUNC PyInit__torch_ops() {
+  PyObject* module = PyModule_Create(&g_module);
+  if (module != nullptr && PyModule_AddStringConstant(module, "source_hash", ATTN_B200_OPS_HASH) != 0) Py_CLEAR(module);
+  return module;
+}

@@ -15,11 +15,10 @@ import threading
 
 import torch
 
-from .. import _lib
+from .. import _lib, build
 from ..autotuner.base_tunner import cache_dir
 from ..autotuner.runtime import KernelError, Runtime
 from ..autotuner.tunner import AttnTunner, RetBwdTunner, RetTunner, is_decoding
-from ..build import OPS_PATH
 
 _ENV = ["ATTN_B200_CACHE_DIR", "ATTN_B200_AUTOTUNE"]
 TRIES = 16  # attempts at a call that no change of the tuning cache overtakes; each change costs one
@@ -35,18 +34,23 @@ def _address(fn) -> int:
 
 
 def ops():
-    """The native module; raises if it has not been built (python -m attention_autotuner_b200.build)."""
+    """The native module; raises if it has not been built from the present sources (python -m attention_autotuner_b200.build)."""
     global _module
     if _module is not None:
         return _module
     with _lock:
         if _module is None:
-            if not os.path.exists(OPS_PATH):
-                raise RuntimeError(f"{OPS_PATH} is missing: build it with `python -m attention_autotuner_b200.build`. "
+            path = build.OPS_PATH
+            if not os.path.exists(path):
+                raise RuntimeError(f"{path} is missing: build it with `python -m attention_autotuner_b200.build`. "
                                    "There is no fallback.")
-            loader = importlib.machinery.ExtensionFileLoader("_torch_ops", OPS_PATH)
+            loader = importlib.machinery.ExtensionFileLoader("_torch_ops", path)
             mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_torch_ops", loader))
             loader.exec_module(mod)
+            if getattr(mod, "source_hash", None) != build._ops_hash():
+                # it calls the C entry points by signatures of its own: a stale one would call them with wrong arguments
+                raise RuntimeError(f"{path} was built from other sources or for another PyTorch: build it again with "
+                                   "`python -m attention_autotuner_b200.build`")
             lib = _lib.load()
             mod.init(KernelError, _lib.AttnB200Error, _resolve_bwd, _address(lib.attn_b200_last_error),
                      _address(lib.attn_b200_fa_bwd), _address(lib.attn_b200_ret_chunk_workspace_bytes),

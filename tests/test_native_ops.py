@@ -26,6 +26,18 @@ def test_plan_goes_stale_with_its_files_and_environment(tmp_path, monkeypatch):
     assert not native.plan_fresh(None)
 
 
+def test_an_extension_made_from_something_else_is_refused(monkeypatch):
+    from attention_autotuner_b200 import build
+    from attention_autotuner_b200.ops import _native
+    module = _native.ops()
+    monkeypatch.setattr(_native, "_module", None)
+    assert type(_native.ops()) is type(module)
+    monkeypatch.setattr(_native, "_module", None)
+    monkeypatch.setattr(build, "_ops_hash", lambda: "0")
+    with pytest.raises(RuntimeError, match="other sources"):
+        _native.ops()
+
+
 def test_a_plan_reads_the_environment_under_the_gil(monkeypatch):
     """os.environ assignments of other threads run setenv under the GIL, so getenv has to as well. A plan with many variables,
     the last one changed: no other thread gets to run while the call looks at them and declines."""
