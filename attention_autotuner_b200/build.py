@@ -10,6 +10,7 @@ import os
 import shutil
 import subprocess
 import sys
+import threading
 
 CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc")
 LIB_PATH = os.environ.get("ATTN_B200_LIB", os.path.join(CSRC, "libattn_b200.so"))  # override: a library built elsewhere
@@ -114,11 +115,15 @@ def build_torch_ops(force: bool = False) -> str:
     torch_dir = os.path.dirname(torch.__file__)
     incs = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
             os.path.join(cuda_home, "include"), sysconfig.get_paths()["include"]]
+    tmp = f"{OPS_PATH}.{os.getpid()}.{threading.get_ident()}.tmp"  # put in place whole: other processes load it, or build it too
     cmd = ["g++", *OPS_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DATTN_B200_OPS_HASH="{want}"',
-           *[f"-I{d}" for d in incs], OPS_SRC, "-o", OPS_PATH, f"-L{os.path.join(torch_dir, 'lib')}", *OPS_LIBS]
+           *[f"-I{d}" for d in incs], OPS_SRC, "-o", tmp, f"-L{os.path.join(torch_dir, 'lib')}", *OPS_LIBS]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
+        if os.path.exists(tmp):
+            os.remove(tmp)
         raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
+    os.replace(tmp, OPS_PATH)
     with open(stamp, "w") as f:
         f.write(want + "\n")
     return OPS_PATH

@@ -38,6 +38,33 @@ def test_an_extension_made_from_something_else_is_refused(monkeypatch):
         _native.ops()
 
 
+def test_a_build_replaces_the_extension_whole_or_not_at_all(monkeypatch, tmp_path):
+    import subprocess
+
+    from attention_autotuner_b200 import build
+    path = tmp_path / "_torch_ops.so"
+    path.write_text("old")
+    monkeypatch.setattr(build, "OPS_PATH", str(path))
+    for status, left in ((1, "old"), (0, "new")):
+        def compiler(cmd, **_k):
+            out = cmd[cmd.index("-o") + 1]
+            with open(out, "w") as f:
+                f.write("half")
+            assert path.read_text() == "old"  # what another process would load now
+            with open(out, "w") as f:
+                f.write("new")
+            return subprocess.CompletedProcess(cmd, status, "", "")
+
+        monkeypatch.setattr(build.subprocess, "run", compiler)
+        if status:
+            with pytest.raises(RuntimeError):
+                build.build_torch_ops()
+        else:
+            build.build_torch_ops()
+        assert path.read_text() == left
+        assert sorted(os.listdir(tmp_path)) == ["_torch_ops.so"] + ([] if status else ["_torch_ops.so.srchash"])
+
+
 def test_a_plan_reads_the_environment_under_the_gil(monkeypatch):
     """os.environ assignments of other threads run setenv under the GIL, so getenv has to as well. A plan with many variables,
     the last one changed: no other thread gets to run while the call looks at them and declines."""
