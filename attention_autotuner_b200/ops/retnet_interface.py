@@ -85,7 +85,32 @@ def RetNetAttnFunc(q, k, v, mask, device_type, causal=False, scale=None, decay=N
     return _call(go, device_type, q, k, v, mask, causal, scale, decay)
 
 
-class RetNetAttn:
-    """The reference's autograd class (python/ops/retnet_interface.py:8-55); its node is native here
-    (csrc/host/torch_ops.cpp: RetNode)."""
-    apply = staticmethod(RetNetAttnFunc)
+class RetNetAttn(torch.autograd.Function):
+    """The reference's autograd class (python/ops/retnet_interface.py:8-55). Its ``apply`` goes through the native node
+    (csrc/host/torch_ops.cpp: RetNode); ``forward`` and ``backward`` are that node's for classes derived from this one."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, mask, device_type, *opts):
+        causal = bool(opts[0]) if len(opts) > 0 else False
+        scale = opts[1] if len(opts) > 1 else None
+        decay = opts[2] if len(opts) > 2 else None
+        q, k, v = [x.contiguous() for x in [q, k, v]]
+        o, r, maskr, decayr = retnet_forward(q, k, v, mask, device_type, causal, scale, decay)
+        ctx.save_for_backward(q, k, v, maskr, r, decayr)
+        ctx.device_type = device_type
+        ctx.opts = (causal, scale)
+        ctx.n_extra = len(opts)
+        return o
+
+    @staticmethod
+    def backward(ctx, do):
+        q, k, v, mask, r, decay = ctx.saved_tensors
+        causal, scale = ctx.opts
+        dq, dk, dv = retnet_backward(q, k, v, mask, do, r, ctx.device_type, causal, scale, decay)
+        return (dq, dk, dv, None, None) + (None,) * ctx.n_extra
+
+    @classmethod
+    def apply(cls, *args, **kwargs):
+        if cls is RetNetAttn:
+            return RetNetAttnFunc(*args, **kwargs)
+        return super().apply(*args, **kwargs)

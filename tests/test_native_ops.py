@@ -127,6 +127,59 @@ def test_declines_what_the_python_checks_word():
             call()
 
 
+def test_the_operators_classes_are_autograd_functions_to_derive_from():
+    from attention_autotuner_b200.ops.attention_interface import MultiHeadAttnFunc
+    from attention_autotuner_b200.ops.retnet_interface import RetNetAttn
+    for base in (MultiHeadAttnFunc, RetNetAttn):
+        assert issubclass(base, torch.autograd.Function)
+
+        class Derived(base):
+            @staticmethod
+            def forward(ctx, x):
+                return 2 * x
+
+            @staticmethod
+            def backward(ctx, g):
+                return 3 * g
+
+        x = torch.ones(2, requires_grad=True)
+        y = Derived.apply(x)
+        y.sum().backward()
+        assert torch.equal(y, torch.full((2,), 2.0)) and torch.equal(x.grad, torch.full((2,), 3.0))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["attention", "mask", "decay"])
+def test_a_derived_class_computes_what_the_operator_does(form):
+    from attention_autotuner_b200.arch import B200
+    from attention_autotuner_b200.ops.attention_interface import MultiHeadAttnFunc, flash_attn_func
+    from attention_autotuner_b200.ops.retnet_interface import RetNetAttn, RetNetAttnFunc
+    q, k, v, do = (torch.randn(1, 64, 2, 64, device="cuda").half().transpose(1, 2) for _ in range(4))
+    if form == "attention":
+        base, func, args = MultiHeadAttnFunc, flash_attn_func, (B200(), True, 0.125)
+    elif form == "mask":
+        base, func, args = RetNetAttn, RetNetAttnFunc, (torch.rand(2, 64, 64, device="cuda").half().tril(), B200(), True)
+    else:
+        base, func, args = RetNetAttn, RetNetAttnFunc, (None, B200(), True, 0.125, torch.tensor([0.97, 0.99]))
+
+    class Derived(base):
+        pass
+
+    results = []
+    for call in (func, base.apply, Derived.apply):
+        leaves = [t.detach().requires_grad_(True) for t in (q, k, v)]
+        o = call(*leaves, *args)
+        results.append((o.detach(), *torch.autograd.grad(o, leaves, do)))
+        with torch.no_grad():
+            assert torch.equal(call(*leaves, *args), o)
+    for other in results[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(results[0], other))
+    if form == "attention":
+        o, lse = Derived.apply(q.detach().requires_grad_(True), k, v, *args, True)
+        assert o.requires_grad and not lse.requires_grad
+        assert torch.equal(lse, flash_attn_func(q, k, v, *args, True)[1])
+
+
 @pytest.mark.gpu
 def test_backward_errors_keep_their_class_and_strided_gradients_are_taken():
     from attention_autotuner_b200.arch import B200
