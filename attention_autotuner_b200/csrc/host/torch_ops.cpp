@@ -28,6 +28,7 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include <cstdlib>
+#include <initializer_list>
 #include <string>
 #include <utility>
 #include <vector>
@@ -319,11 +320,12 @@ struct RetNode : public torch::autograd::Function<RetNode> {
 };
 
 // ------------------------------------------------------------------------------------------------ Python functions
-// Whether the call has to go through an autograd node. Forward-mode duals do too, whatever the grad mode: the node raises
-// (there is no jvp), whereas the plain launch would drop the tangents.
-bool any_grad(const Tensor& a, const Tensor& b, const Tensor& c) {
-  for (const Tensor* t : {&a, &b, &c})
-    if (t->_fw_grad(/*level=*/0).defined() || (at::GradMode::is_enabled() && t->requires_grad())) return true;
+// Whether the call has to go through an autograd node: any of its tensors does, the mask or the decay as well (their gradient
+// is none, but the output has a node). Forward-mode duals do too, whatever the grad mode: the node raises (there is no jvp),
+// whereas the plain launch would drop the tangents.
+bool any_grad(std::initializer_list<const Tensor*> tensors) {
+  for (const Tensor* t : tensors)
+    if (t->defined() && (t->_fw_grad(/*level=*/0).defined() || (at::GradMode::is_enabled() && t->requires_grad()))) return true;
   return false;
 }
 // A tensor argument, or an undefined tensor for None; false for any other object.
@@ -361,7 +363,7 @@ PyObject* py_attn(PyObject*, PyObject* const* a, Py_ssize_t n) {
   {
     py::gil_scoped_release nogil;
     if (!plan->files_unchanged()) plan = nullptr;
-    else if (any_grad(q, k, v)) {
+    else if (any_grad({&q, &k, &v})) {
       variable_list out = AttnNode::apply(q, k, v, reinterpret_cast<int64_t>(plan), scale, causal != 0, ret_lse != 0);
       o = out[0];
       if (ret_lse) lse = out[1];
@@ -398,7 +400,7 @@ PyObject* py_retnet(PyObject*, PyObject* const* a, Py_ssize_t n) {
   {
     py::gil_scoped_release nogil;
     if (!plan->files_unchanged()) plan = nullptr;
-    else if (any_grad(q, k, v)) {
+    else if (any_grad({&q, &k, &v, &mask, &decay})) {
       auto given = [](const Tensor& t) { return t.defined() ? std::optional<Tensor>(t) : std::nullopt; };
       o = RetNode::apply(q, k, v, given(mask), given(decay), reinterpret_cast<int64_t>(plan), reinterpret_cast<int64_t>(bwd),
                          static_cast<int64_t>(token), scale, causal != 0)[0];

@@ -224,3 +224,32 @@ def test_forward_mode_duals_are_refused_not_dropped():
             flash_attn_func(d, k, v, B200(), True, 0.125)
         with pytest.raises(RuntimeError):
             RetNetAttnFunc(k, d, v, None, B200(), True, 0.125, torch.tensor([0.97, 0.99]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["mask", "decay"])
+def test_a_mask_or_decay_alone_takes_the_call_through_the_node(form):
+    import torch.autograd.forward_ad as fwAD
+    from attention_autotuner_b200.arch import B200
+    from attention_autotuner_b200.ops.retnet_interface import RetNetAttnFunc
+    q, k, v = (torch.randn(1, 2, 64, 64, device="cuda").half() for _ in range(3))
+    factor = torch.rand(2, 64, 64, device="cuda").half() if form == "mask" else torch.tensor([0.97, 0.99], device="cuda")
+
+    def call(f, q=q):
+        return RetNetAttnFunc(q, k, v, f, B200(), False, 0.125) if form == "mask" else RetNetAttnFunc(q, k, v, None, B200(), True, 0.125, f)
+
+    want = call(factor)
+    assert not want.requires_grad
+    with fwAD.dual_level(), pytest.raises(RuntimeError):
+        call(fwAD.make_dual(factor, torch.ones_like(factor)))
+    learned = factor.clone().requires_grad_(True)
+    got = call(learned)
+    assert got.requires_grad and torch.equal(got, want)
+    # the gradient of q is that of a constant mask or decay; the factor itself gets none
+    do = torch.randn_like(want)
+    qg, qh = (q.clone().requires_grad_(True) for _ in range(2))
+    call(learned, qg).backward(do)
+    call(factor, qh).backward(do)
+    assert torch.equal(qg.grad, qh.grad) and learned.grad is None
+    with torch.no_grad():
+        assert not call(learned).requires_grad
