@@ -1,6 +1,6 @@
 """The order of work of the persistent kernels (csrc/work_order.cuh), compiled for the host: in each order every (row
 block, slice) is taken exactly once, whatever the number of workers, and the chosen order loads no worker more than pairs
-of row blocks would."""
+of row blocks would, under a causal mask and without one; and the limit on the operands in flight."""
 import subprocess
 
 from attention_autotuner_b200.build import CSRC
@@ -12,8 +12,9 @@ PROGRAM = r"""
 #include <cstdio>
 #include <vector>
 using namespace ab200;
-// most loaded worker, or -1 if an item is missed, taken twice or out of range; items of rank k cost nrb - k
-static long run(const WorkList& w, int slices, int workers) {
+// most loaded worker, or -1 if an item is missed, taken twice or out of range; items of rank k cost nrb - k under a causal
+// mask (triangular), all the same without one
+static long run(const WorkList& w, int slices, int workers, bool triangular = true) {
   std::vector<char> seen(static_cast<size_t>(w.nrb) * slices, 0);
   long worst = 0;
   size_t n = 0;
@@ -23,7 +24,7 @@ static long run(const WorkList& w, int slices, int workers) {
       int k = -1, s = -1;
       if (!w.step(u, c, workers, k, s)) continue;
       if (k < 0 || k >= w.nrb || s < 0 || s >= slices || seen[static_cast<size_t>(s) * w.nrb + k]++) return -1;
-      load += w.nrb - k;
+      load += triangular ? w.nrb - k : 1;
       ++n;
     }
     if (load > worst) worst = load;
@@ -42,6 +43,24 @@ int main() {
     }
     const int pick = pick_work_order(sl, nrb, full, true, 1e3);
     if (load[pick] > load[kOrderPairs]) { printf("pick nrb %d slices %d workers %d\n", nrb, sl, full); return 1; }
+    // operands of the slices in flight beyond half of L2: pairs, whatever the balance
+    const int in_flight = sl < full ? sl : full;
+    if (pick_work_order(sl, nrb, full, true, 51e6 / in_flight) != kOrderPairs ||
+        pick_work_order(sl, nrb, full, true, 49e6 / in_flight) != pick) {
+      printf("limit nrb %d slices %d workers %d\n", nrb, sl, full);
+      return 1;
+    }
+    // equal costs: slice after slice or in pairs, whichever loads the busiest worker least
+    const int flat = pick_work_order(sl, nrb, full, false, 1e9);
+    long even[2];
+    for (int order : {kOrderSlices, kOrderPairs}) {
+      const WorkList w = work_list(order, sl, nrb);
+      even[order] = run(w, sl, w.units < full ? w.units : full, false);
+    }
+    if (flat > kOrderPairs || even[flat] != (even[0] < even[1] ? even[0] : even[1])) {
+      printf("flat nrb %d slices %d workers %d\n", nrb, sl, full);
+      return 1;
+    }
   }
   return 0;
 }
