@@ -1,7 +1,7 @@
 // flash-attention forward for a handful of query rows (decoding: up to 16 new positions against a long K / V cache).
 //
-// What bounds it: reading K and V once. 16 rows give 32 FLOP per byte of K and V, a tenth of what the tensor cores need to
-// be the limit, so the tile of 128 query rows of fa_fwd_sm100.cuh does nothing but fetch: one CTA per (batch, head) slice,
+// What bounds it: reading K and V once. A key costs 64 d FLOP with 16 rows and 4 d bytes, 16 FLOP per byte of K and V, a
+// sixteenth of what the tensor cores need to be the limit (1640 TFLOP/s over 6.53 TB/s), so the tile of 128 query rows of fa_fwd_sm100.cuh does nothing but fetch: one CTA per (batch, head) slice,
 // one block of 128 keys (64 KB) per 1.8 us of serial S -> softmax -> P V chain. Here
 //   * the keys of a slice are split over the CTAs of a thread-block cluster (1, 4 or 8, by the number of keys); each keeps its own maximum, sum and accumulator, and the cluster combines them through
 //     distributed shared memory at the end: one launch, no scratch memory;

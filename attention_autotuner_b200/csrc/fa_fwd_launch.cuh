@@ -126,16 +126,16 @@ int fa_fwd_persist_launch(const FaFwdArgs& a, cudaStream_t stream) {
 }
 
 // Launcher of the decoding kernel (up to 16 query rows, head dimensions 64 and 128, the same for q, k and v).
-// nsplit = CTAs (a cluster) per slice; 0: chosen here, by the number of blocks alone: the order in which a slice's partial
-// results are added, and so its output to the last bit, must not depend on how many other slices are in the launch
-// (sharding by slices gives the same bits on any number of ranks). Measured at d = 128, 1 / 4 / 8 CTAs: BH = 32, Lkv = 16384:
+// CTAs (a cluster) per slice are chosen by the number of blocks alone: the order in which a slice's partial results are
+// added, and so its output to the last bit, must not depend on how many other slices are in the launch (sharding by slices
+// gives the same bits on any number of ranks). Measured at d = 128, 1 / 4 / 8 CTAs: BH = 32, Lkv = 16384:
 // 117 / 45.1 / 45.2 us; BH = 16, Lkv = 32768: 223 / 65 / 46.9; BH = 64, Lkv = 8192: 64.6 / 44.6 / 47.2; BH = 256, Lkv = 4096:
 // 80.0 / 82.8 / 91; BH = 512, Lkv = 2048: 79.6 / 87 / 114, Lkv = 256: 18.5 / 36 / 70. Four lose little with many slices and
 // win most of what there is with few; eight where a cache is long enough to hide the larger cluster.
 inline int fa_decode_split(int nblk) { return nblk >= 256 ? 8 : nblk >= 32 ? 4 : 1; }
 
 template <int D, bool BF16>
-int fa_decode_launch(const FaFwdArgs& a, cudaStream_t stream, int nsplit = 0) {
+int fa_decode_launch(const FaFwdArgs& a, cudaStream_t stream) {
   using Cfg = FaDecodeConfig<D, BF16>;
   if (!a.q || !a.k || !a.v || !a.o) return fail(kErrInvalidArgument, "fa_fwd: null tensor pointer");
   if (a.BH <= 0 || a.Lq <= 0 || a.Lkv <= 0) return fail(kErrInvalidArgument, "fa_fwd: sizes must be positive");
@@ -162,7 +162,7 @@ int fa_decode_launch(const FaFwdArgs& a, cudaStream_t stream, int nsplit = 0) {
   auto kernel = &fa_decode_sm100_kernel<Cfg>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES);
   if (e != cudaSuccess) return fail(kErrCuda, "fa_fwd: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  const int c = nsplit > 0 ? nsplit : fa_decode_split((a.Lkv + Cfg::BN - 1) / Cfg::BN);
+  const int c = fa_decode_split((a.Lkv + Cfg::BN - 1) / Cfg::BN);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(c, 1, a.BH);
   cfg.blockDim = dim3(Cfg::NTHREADS, 1, 1);

@@ -10,9 +10,10 @@
 //                 is then made of the lightest items. A worker's neighbours are on other slices, so operands are re-read
 //                 from DRAM if those of the slices in flight do not fit in L2.
 // Measured: RetNet forward B=1 H=8 L=500 (dqk 256, dv 512; 32 items, 16 pairs, 74 CTA pairs) 20.5 us a pass with pairs, 14.4 to
-// 15.7 with the items one by one. The attention kernels keep their pairs: at their sizes with many items per SM the power
-// cap, not the busiest SM, sets the time (a snake order cost the forward 4 %), with few the forward has other forms, and in
-// the backward even the same order through this structure cost the dQ kernel 5 % (B=8 H=32 L=1795 d=64: 442 -> 466 us).
+// 15.7 with the items one by one. The attention kernels do not use this structure. The persistent forward keeps its pairs (a
+// snake order cost it 4 %: spills in the softmax loop, K and V of all slices in flight out of L2) and leaves the shapes that
+// pairs balance badly to its grid form. In the backward the order evaluated at run time cost the dQ kernel 5 % (B=8 H=32 L=1795
+// d=64: 442 -> 466 us), so its single blocks are a specialisation of the kernels (fa_bwd_singles).
 #pragma once
 
 namespace ab200 {
