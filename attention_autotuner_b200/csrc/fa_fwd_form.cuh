@@ -1,0 +1,68 @@
+// Which form of the grid serves an attention forward of 256-row items: a rule on sizes alone, also compiled for the host by
+// its test.
+#pragma once
+
+namespace ab200 {
+
+// Time of both forms in units of one KV block of one item (128 keys against 256 rows, about 2.1 us at d = 128), as the busiest
+// SM spends it:
+//   * grid form: a CTA per item, given out as SMs become free. An item costs its blocks and 2.6 more for set-up and epilogue.
+//     Items of equal cost: rounds of them. Under a causal mask they run from `first` to `last` blocks (heaviest ones first):
+//     the mean load of an SM and 0.6 of the heaviest item, but no more than rounds of the heaviest.
+//   * persistent form: one CTA per SM, pairs (heaviest with lightest item of a slice; the middle one of an odd count alone)
+//     dealt in turn. What overlaps between items leaves 1.0 per item, and 2.0 once per launch. The busiest SM has only pairs,
+//     unless the deal moves by one position of the slice's list per round (sms and the list's length without a common
+//     factor), as it does with one item per slice: then its share of middle items.
+// Constants fitted to 292 measurements of both forms (B200; 10 to 2000 slices, Lq 64 to 4500, Lkv to 4096, d = 64 and 128, with
+// and without a mask): the form picked is 0.1 % slower than the faster one on average, 10 % at worst (148 slices of L=700, d=64
+// causal, 41.1 / 45.0 us). Comparing the rounds of pairs with those of items instead, whatever the blocks of an item, cost 4.6 %
+// on average and up to 42 %: with one item per slice both forms hold the same items, and short items gain most at
+// their boundaries.
+// Measured grid / persistent in us, without a mask (causal); d = 128 where not stated:
+//   persistent:  2000 slices of L=64 74.3 / 53.3 (75.4 / 53.3), 1000 of L=256 73.3 / 58.3, d=64 55.3 / 43.7 (59.4 / 47.1),
+//                400 of L=256 32.7 / 25.1, 512 of L=512 108.9 / 101.3 (93.9 / 80.6), 96 of L=1300 108.5 / 104.5 (85.1 / 75.5),
+//                12 of L=5000 164 / 164 (122 / 90), 148 of L=2048 +5 % (+18 %), 128 of L=4096 +1 % (+8 %)
+//   grid:        8 of L=512 d=64 12.3 / 19.1, 40 of L=2048 106.8 / 135.5 (71.5 / 84.0), 20 of L=4000 197.6 / 260 (122.7 / 144),
+//                52 of L=1280 51 / 90 (46 / 61), 100 of L=700 51.0 / 61.4 (35.2 / 49.2), 60 of L=2700 253.6 / 302.0
+//                (153.9 / 160.9), 200 of L=768 91.7 / 94.6 (65.7 / 73.8)
+//   one each:    100 of L=1792 grid 168.5 / 185.2 (persistent 117.4 / 114.6)
+struct FaFormCost {
+  double grid, persistent;
+};
+
+inline FaFormCost fa_form_cost(long long slices, int Lq, int Lkv, bool causal, int sms) {
+  const long long nqb = (Lq + 255ll) / 256, nblk = (Lkv + 127ll) / 128, shift = static_cast<long long>(Lkv) - Lq;
+  auto blocks = [&](long long item) -> double {  // KV blocks its last row sees
+    if (!causal) return static_cast<double>(nblk);
+    const long long keys = 256 * (item + 1) + shift, n = keys > 0 ? (keys + 127) / 128 : 0;
+    return static_cast<double>(n < nblk ? n : nblk);
+  };
+  const double first = blocks(0), last = blocks(nqb - 1), mean = 0.5 * (first + last);
+  const long long items = slices * nqb, rounds = (items + sms - 1) / sms;
+  const double even = static_cast<double>(rounds) * (first + 2.6), heavy = static_cast<double>(rounds) * (last + 2.6),
+               spread = static_cast<double>(items) / sms * (mean + 2.6) + 0.6 * (last + 2.6);
+  const double uneven = heavy < spread ? heavy : spread;
+
+  const long long npair = (nqb + 1) / 2, units = (slices * npair + sms - 1) / sms;
+  long long a = sms, b = npair;  // greatest common divisor
+  while (b != 0) {
+    const long long r = a % b;
+    a = b;
+    b = r;
+  }
+  const long long middles = (nqb % 2 != 0 && a == 1) ? units / npair : 0;
+  return FaFormCost{even > uneven ? even : uneven,
+                    static_cast<double>(units - middles) * (first + last + 2.0) + static_cast<double>(middles) * (mean + 1.0) + 2.0};
+}
+
+// Long items (more than 40 KV blocks on average) take the grid form whatever the count: a static work list loses more to the
+// slowest SM than the boundaries cost. Without a mask / under a causal one, persistent against grid: L = 8192 0 % / +3 %,
+// B=16 H=32 L=16384 -2 % / -2 %, Lq=1024 x Lkv=16384 -3 %.
+inline bool fa_form_persistent(long long slices, int Lq, int Lkv, bool causal, int sms) {
+  const int nblk = (Lkv + 127) / 128;
+  if ((causal ? (nblk + 1) / 2 : nblk) > 40) return false;
+  const FaFormCost c = fa_form_cost(slices, Lq, Lkv, causal, sms);
+  return c.persistent < c.grid;
+}
+
+}  // namespace ab200

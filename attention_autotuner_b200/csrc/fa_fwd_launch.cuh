@@ -8,6 +8,7 @@
 #include <stdlib.h>
 
 #include "fa_decode_sm100.cuh"
+#include "fa_fwd_form.cuh"
 #include "fa_fwd_pair_sm100.cuh"
 #include "fa_fwd_persist_sm100.cuh"
 #include "fa_fwd_sm100.cuh"
@@ -180,28 +181,15 @@ int fa_decode_launch(const FaFwdArgs& a, cudaStream_t stream) {
   return check_launch("fa_fwd launch");
 }
 
-// The default tile (two query tiles, up to 128 V columns, no softmax variant) exists in both forms; the persistent one
-// runs where a CTA's work items are short, because what it saves lies at their boundaries. Measured against the grid
-// form in one session (d = 128, back-to-back launches), without a mask / under a causal one: 148 slices of L = 2048
-// +5 % / +18 %, B=8 H=16 L=4096 +1 % / +8 %, L = 8192 0 % / +3 %, B=16 H=32 L=16384 -2 % / -2 %, Lq=1024 x Lkv=16384
-// -3 % (with long items a static work list loses more to the slowest SM than the boundaries cost). The rule: persistent
-// up to 40 KV blocks per item on average (half of the blocks count under a causal mask), unless dealing pairs of items puts
-// clearly more of them on the busiest SM than one at a time would (a quarter more under a causal mask, where the grid form
-// gives up more at the items' boundaries, a tenth more without one).
-// Measured grid / persistent, bf16, 2 x rounds of pairs against rounds of items: 4 : 3, BH=40 L=2048 d=128 106.8 / 135.5 us
-// (causal 71.5 / 84.0), BH=100 L=700 49.6 / 61.5 (36.1 / 51.2), BH=20 L=4000 197.6 / 260 (122.7 / 144); 4 : 2, BH=52 L=1280
-// 51 / 90 (46 / 61); 6 : 5, BH=60 L=2700 253.6 / 302.0 (153.9 / 160.9), BH=100 L=1792 168.5 / 185.2 (117.4 / 114.6); 2 : 1, BH=8 L=512 d=64 12.3 / 19.1; 2 : 2, BH=12 L=5000 164 / 164 (122 / 90); 4 : 4, BH=96 L=1300
-// 108.5 / 104.5 (85.1 / 75.5).
+// The default tile (two query tiles, up to 128 V columns, no softmax variant) exists in both forms, with the same bits; what
+// the persistent one saves lies at the boundaries of the work items. fa_fwd_form.cuh has the rule.
 template <class Cfg>
 bool fa_fwd_picks_persistent(const FaFwdArgs& a) {
   if constexpr (Cfg::NQ == 2 && Cfg::SPLIT == 1 && Cfg::NMMA == 1 && Cfg::EXP_EMU == 0 && Cfg::EXP_H2 == 0 && Cfg::DV <= 128) {
+    static_assert(Cfg::NQ * Cfg::BM == 256 && Cfg::BN == 128, "the rule's items and blocks");
     const int form = fa_fwd_form_requested();
-    const int nblk = (a.Lkv + Cfg::BN - 1) / Cfg::BN;
-    const int avg_blocks = a.causal ? (nblk + 1) / 2 : nblk;
-    const long long nqb = (a.Lq + 2 * Cfg::BM - 1) / (2 * Cfg::BM), slices = static_cast<long long>(a.BH) * (a.dv / Cfg::DV);
-    const long long sms = sm_count(), pair_rounds = (slices * ((nqb + 1) / 2) + sms - 1) / sms, item_rounds = (slices * nqb + sms - 1) / sms;
-    const bool coarse = a.causal ? 4 * 2 * pair_rounds >= 5 * item_rounds : 10 * 2 * pair_rounds >= 11 * item_rounds;
-    return form == 2 || (form == 0 && avg_blocks <= 40 && !coarse);
+    const long long slices = static_cast<long long>(a.BH) * (a.dv / Cfg::DV);
+    return form == 2 || (form == 0 && fa_form_persistent(slices, a.Lq, a.Lkv, a.causal != 0, sm_count()));
   }
   return false;
 }
