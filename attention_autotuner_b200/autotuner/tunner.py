@@ -22,14 +22,11 @@ def _flops_fwd(t, causal):
     return 2.0 * B * H * pairs * (dqk + dv)
 
 
-# What csrc/fa_fwd_launch.cuh (fa_fwd_is_decode) sends to the decoding kernel: up to DECODE_ROWS query rows, one head
-# dimension out of DECODE_DIMS for q, k and v, and no form of the grid asked for in the environment.
-DECODE_ROWS = 16
-DECODE_DIMS = (64, 128)
-
-
 def is_decoding(q_shape, v_shape) -> bool:
-    return (q_shape[-2] <= DECODE_ROWS and q_shape[-1] == v_shape[-1] and q_shape[-1] in DECODE_DIMS
+    """What csrc/fa_fwd_launch.cuh (fa_fwd_is_decode) sends to the decoding kernel: the shapes of fa_decode_shape
+    (csrc/fa_fwd_form.cuh), unless a form of the grid is asked for in the environment."""
+    Lq, d, Lkv = q_shape[-2], q_shape[-1], v_shape[-2]
+    return (Lq <= 16 and d == v_shape[-1] and (d == 64 or (d == 128 and (Lq <= 12 or Lkv > 256)))
             and os.environ.get("ATTN_B200_FA_FWD_FORM", "")[:1] not in ("g", "p"))
 
 

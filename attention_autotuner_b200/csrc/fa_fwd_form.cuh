@@ -1,8 +1,21 @@
-// Which form of the grid serves an attention forward of 256-row items: a rule on sizes alone, also compiled for the host by
-// its test.
+// Which kernel, and which form of the grid, serves an attention forward: rules on sizes alone, also compiled for the host by
+// their tests.
 #pragma once
 
 namespace ab200 {
+
+// The decoding kernel (fa_decode_sm100.cuh): one head dimension of 64 or 128 for q, k and v and up to 16 query rows, the rows of
+// its tile. At d = 128 its warps' partial rows are added at the end at a cost that grows with the rows, which a few keys do
+// not hide: more than 12 rows with up to 256 keys stay on the large tile. Decoding kernel / large tile in us, bf16, 1, 148 and
+// 2048 slices: Lq = 16, Lkv = 128 9.8 / 7.2, 10.2 / 8.2, 69.6 / 55.3; Lq = 16, Lkv = 256 10.2 / 8.2, 10.2 / 10.2, 85.3 / 77.8 (but
+// 512 slices 22.5 / 26.1); Lq = 16, Lkv = 512 12.3 / 12.3, 12.3 / 13.4, 115 / 130; Lq = 12, Lkv = 128 8.2 / 7.2, 8.2 / 8.2, 59.4 / 55.3, Lkv = 256
+// 9.2 / 8.2, 10.2 / 10.2, 75.5 / 77.8. With 8 rows, and at d = 64 with any, it is the faster one or at most 1 us behind at every
+// size measured (1 to 2048 slices, 16 to 4096 keys). The number of slices has no part in the rule: a slice has the same
+// bits in any launch.
+inline bool fa_decode_shape(int dqk, int dv, int Lq, int Lkv) {
+  if (dv != dqk || Lq > 16) return false;
+  return dqk == 64 || (dqk == 128 && (Lq <= 12 || Lkv > 256));
+}
 
 // Time of both forms in units of one KV block of one item (128 keys against 256 rows, about 2.1 us at d = 128), as the busiest
 // SM spends it:

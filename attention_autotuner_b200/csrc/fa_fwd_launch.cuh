@@ -194,11 +194,9 @@ bool fa_fwd_picks_persistent(const FaFwdArgs& a) {
   return false;
 }
 
-// Up to 16 query rows with one head dimension of 64 or 128: faster at every size measured (BH 1 to 512, Lkv 256 to 32768),
-// since the large tile works on 256 rows whatever it is given. The tile's row count is the limit.
 template <class Cfg>
 bool fa_fwd_is_decode(const FaFwdArgs& a) {
-  return (Cfg::DQK == 64 || Cfg::DQK == 128) && a.dv == Cfg::DQK && a.Lq <= 16 && fa_fwd_form_requested() == 0;
+  return fa_decode_shape(Cfg::DQK, a.dv, a.Lq, a.Lkv) && fa_fwd_form_requested() == 0;
 }
 
 template <class Cfg>

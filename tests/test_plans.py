@@ -4,6 +4,7 @@ cache, and kept apart from that of longer calls."""
 import json
 import os
 import re
+import subprocess
 
 import pytest
 import torch
@@ -15,9 +16,9 @@ from attention_autotuner_b200.autotuner.tunner import AttnTunner
 from attention_autotuner_b200.build import CSRC
 
 
-def tensors(Lq, d, dv=None, dt=torch.bfloat16):
-    q, k = torch.zeros(1, 2, Lq, d, dtype=dt), torch.zeros(1, 2, 64, d, dtype=dt)
-    return [q, k, torch.zeros(1, 2, 64, dv or d, dtype=dt), torch.zeros(1, 2, Lq, dv or d, dtype=dt)]
+def tensors(Lq, d, dv=None, dt=torch.bfloat16, Lkv=512):
+    q, k = torch.zeros(1, 2, Lq, d, dtype=dt), torch.zeros(1, 2, Lkv, d, dtype=dt)
+    return [q, k, torch.zeros(1, 2, Lkv, dv or d, dtype=dt), torch.zeros(1, 2, Lq, dv or d, dtype=dt)]
 
 
 class Searched(Exception):
@@ -162,11 +163,27 @@ def test_an_operator_prepares_again_what_a_change_has_overtaken(monkeypatch):
                     call()
 
 
-def test_the_rule_is_the_launchers():
+PROGRAM = r"""
+#include "fa_fwd_form.cuh"
+#include <cstdio>
+int main() {
+  int dqk, dv, lq, lkv;
+  while (scanf("%d %d %d %d", &dqk, &dv, &lq, &lkv) == 4) printf("%d\n", ab200::fa_decode_shape(dqk, dv, lq, lkv) ? 1 : 0);
+}
+"""
+
+
+def test_the_rule_is_the_launchers(tmp_path):
+    (tmp_path / "rule.cpp").write_text(PROGRAM)
+    subprocess.run(["g++", "-std=c++17", "-I" + CSRC, str(tmp_path / "rule.cpp"), "-o", str(tmp_path / "rule")], check=True)
+    shapes = [(dqk, dv, lq, lkv) for dqk in (64, 128, 192, 256) for dv in (64, 128, 256) for lq in range(1, 19) for lkv in (1, 16, 255, 256, 257, 9000)]
+    out = subprocess.run([str(tmp_path / "rule")], input="\n".join(" ".join(map(str, x)) for x in shapes), capture_output=True, text=True, check=True)
+    got = [x == "1" for x in out.stdout.split()]
+    assert got == [tunner.is_decoding((1, 1, lq, dqk), (1, 1, lkv, dv)) for dqk, dv, lq, lkv in shapes]
+    taken = {x for x, g in zip(shapes, got) if g}
+    # the kernel's tile holds 16 rows; more than 12 with few keys were slower on it at d = 128 (16 rows, 128 keys, 2048 slices:
+    # 69.6 us against 55.3)
     with open(os.path.join(CSRC, "fa_decode_sm100.cuh")) as f:
-        rows = re.search(r"int MAX_ROWS = (\d+);", f.read())
-    with open(os.path.join(CSRC, "fa_fwd_launch.cuh")) as f:
-        rule = re.search(r"bool fa_fwd_is_decode\(.*?\n}", f.read(), re.S).group(0)
-    assert int(rows.group(1)) == tunner.DECODE_ROWS
-    assert [int(x) for x in re.findall(r"Cfg::DQK == (\d+)", rule)] == list(tunner.DECODE_DIMS)
-    assert re.findall(r"a\.Lq <= (\d+)", rule) == [str(tunner.DECODE_ROWS)] and "a.dv == Cfg::DQK" in rule
+        assert max(x[2] for x in taken) <= int(re.search(r"int MAX_ROWS = (\d+);", f.read()).group(1))
+    assert (128, 128, 16, 257) in taken and (128, 128, 12, 16) in taken and (64, 64, 16, 16) in taken
+    assert not {(128, 128, 16, 16), (128, 128, 13, 256)} & taken
