@@ -27,6 +27,7 @@ from __future__ import annotations
 
 import glob
 import json
+import math
 import os
 import re
 
@@ -51,6 +52,25 @@ def parse_config_repr(text: str) -> dict:
         else:
             out[key] = val
     return out
+
+
+def forward_is_persistent(slices: int, Lq: int, Lkv: int, causal: bool, sms: int = SM_COUNT) -> bool:
+    """The launcher's choice between the forms of the forward's grid (csrc/fa_fwd_form.cuh: fa_form_persistent)."""
+    nqb, nblk = -(-Lq // 256), -(-Lkv // 128)
+    if (-(-nblk // 2) if causal else nblk) > 40:
+        return False
+
+    def blocks(item):
+        return min(nblk, max(0, -(-(256 * (item + 1) + Lkv - Lq) // 128))) if causal else nblk
+
+    first, last = blocks(0), blocks(nqb - 1)
+    mean, items = 0.5 * (first + last), slices * nqb
+    rounds = -(-items // sms)
+    grid = max(rounds * (first + 2.6), min(rounds * (last + 2.6), items / sms * (mean + 2.6) + 0.6 * (last + 2.6)))
+    npair = (nqb + 1) // 2
+    units = -(-slices * npair // sms)
+    middles = units // npair if nqb % 2 and math.gcd(sms, npair) == 1 else 0
+    return (units - middles) * (first + last + 2.0) + middles * (mean + 1.0) + 2.0 < grid
 
 
 def _pairs(Lq: int, Lkv: int, causal: bool) -> float:
@@ -89,12 +109,12 @@ def features(op: str, cfg: dict, problem: dict) -> np.ndarray:
         pair = 1.0 if cfg.get("cta_pair", 0) else 0.0
         tiles = problem["B"] * problem["H"] * np.ceil(problem["Lq"] / 128.0) * passes / SM_COUNT / 1e6
         # the persistent form of the grid has no per-CTA prologue / epilogue to pay; left to the launcher (-1) it is
-        # taken up to 40 KV blocks per work item on average (csrc/fa_fwd_launch.cuh)
+        # taken where it is estimated to be the faster one
         persistent = cfg.get("persistent", -1)
         if persistent == -1 and q_tiles == 2 and chunk <= 128 and split == 1 and not cfg.get("exp_emu", 0) \
                 and not cfg.get("exp_h2", 0) and cfg.get("mma_warps", 1) == 1 and not cfg.get("cta_pair", 0):
-            nblk = np.ceil(problem["Lkv"] / 128.0)
-            persistent = 1 if (np.ceil(nblk / 2.0) if problem.get("causal", False) else nblk) <= 40 else 0
+            persistent = int(forward_is_persistent(int(problem["B"] * problem["H"] * passes), int(problem["Lq"]), int(problem["Lkv"]),
+                                                   bool(problem.get("causal", False))))
         if persistent == 1:
             tiles = 0.0
         return np.array([

@@ -1,7 +1,9 @@
 """The rule between the two forms of the attention forward's grid (csrc/fa_fwd_form.cuh), compiled for the host: it takes the
 faster form of measured shapes, and the persistent one wherever slices of one work item each share an SM."""
+import random
 import subprocess
 
+from attention_autotuner_b200.autotuner.cost_model import forward_is_persistent
 from attention_autotuner_b200.build import CSRC
 
 # slices, Lq, Lkv, causal, grid us, persistent us; measured on a B200 (148 SMs) at d = 128, the forms at least 4 % apart
@@ -40,6 +42,11 @@ def test_the_faster_form_is_picked(tmp_path):
            for lkv in (lq, 700, 5000) for c in (0, 1)]
     for call, got in zip(one, persistent(one)):
         assert got == (call[0] > call[4]), call
+    # the cost model's copy of the rule
+    rng = random.Random(1)
+    calls = [(rng.choice((1, 8, 37, 148, 512, 4000)), rng.randint(17, 6000), rng.randint(1, 12000), rng.randint(0, 1), rng.choice((132, 148)))
+             for _ in range(3000)]
+    assert persistent(calls) == [forward_is_persistent(n, lq, lkv, bool(c), sms) for n, lq, lkv, c, sms in calls]
     # long items, rows that see no key, the largest sizes
     edge = [(512, 16384, 16384, 0, 148), (512, 16384, 16384, 1, 148), (4, 2000, 3, 1, 148), (65535, 2 ** 31 - 1, 2 ** 31 - 1, 1, 148)]
     assert persistent(edge)[:2] == [False, False] and len(persistent(edge)) == len(edge)
