@@ -17,7 +17,7 @@ inline bool fa_decode_shape(int dqk, int dv, int Lq, int Lkv) {
   return dqk == 64 || (dqk == 128 && (Lq <= 12 || Lkv > 256));
 }
 
-// Time of both forms in units of one KV block of one item (128 keys against 256 rows, about 2.1 us at d = 128), as the busiest
+// Time of both forms in units of one KV block of one item (128 keys against 256 rows, about 1.8 us at d = 128), as the busiest
 // SM spends it:
 //   * grid form: a CTA per item, given out as SMs become free. An item costs its blocks and 2.6 more for set-up and epilogue.
 //     Items of equal cost: rounds of them. Under a causal mask they run from `first` to `last` blocks (heaviest ones first):
@@ -26,19 +26,20 @@ inline bool fa_decode_shape(int dqk, int dv, int Lq, int Lkv) {
 //     dealt in turn. What overlaps between items leaves 1.0 per item, and 2.0 once per launch. The busiest SM has only pairs,
 //     unless the deal moves by one position of the slice's list per round (sms and the list's length without a common
 //     factor), as it does with one item per slice: then its share of middle items.
-// Constants fitted to 292 measurements of both forms (B200; 10 to 2000 slices, Lq 64 to 4500, Lkv to 4096, d = 64 and 128, with
-// and without a mask): the form picked is 0.1 % slower than the faster one on average, 10 % at worst (148 slices of L=700, d=64
-// causal, 41.1 / 45.0 us). Comparing the rounds of pairs with those of items instead, whatever the blocks of an item, cost 4.6 %
-// on average and up to 42 %: with one item per slice both forms hold the same items, and short items gain most at
-// their boundaries.
+// Constants fitted to 292 measurements of both forms of an earlier kernel, whose products of a tile waited for one another (10 to
+// 2000 slices, Lq 64 to 4500, Lkv to 4096, d = 64 and 128, with and without a mask); over 116 measurements of the present one
+// (5 to 2000 slices, Lq 64 to 16384, Lkv to 16384) the form picked is 0.3 % slower than the faster one on average, 8 % at worst
+// (96 slices of Lq=512, Lkv=4096, d=128). Comparing the rounds of pairs with those of items instead, whatever the blocks of
+// an item, cost 4.6 % on average and up to 42 %: with one item per slice both forms hold the same items, and short items gain
+// most at their boundaries.
 // Measured grid / persistent in us, without a mask (causal); d = 128 where not stated:
-//   persistent:  2000 slices of L=64 74.3 / 53.3 (75.4 / 53.3), 1000 of L=256 73.3 / 58.3, d=64 55.3 / 43.7 (59.4 / 47.1),
-//                400 of L=256 32.7 / 25.1, 512 of L=512 108.9 / 101.3 (93.9 / 80.6), 96 of L=1300 108.5 / 104.5 (85.1 / 75.5),
-//                12 of L=5000 164 / 164 (122 / 90), 148 of L=2048 +5 % (+18 %), 128 of L=4096 +1 % (+8 %)
-//   grid:        8 of L=512 d=64 12.3 / 19.1, 40 of L=2048 106.8 / 135.5 (71.5 / 84.0), 20 of L=4000 197.6 / 260 (122.7 / 144),
-//                52 of L=1280 51 / 90 (46 / 61), 100 of L=700 51.0 / 61.4 (35.2 / 49.2), 60 of L=2700 253.6 / 302.0
-//                (153.9 / 160.9), 200 of L=768 91.7 / 94.6 (65.7 / 73.8)
-//   one each:    100 of L=1792 grid 168.5 / 185.2 (persistent 117.4 / 114.6)
+//   persistent:  2000 slices of L=64 84 / 56 (84 / 56), 1000 of L=256 68 / 53, d=64 57.7 / 40.8 (57.5 / 43.2),
+//                400 of L=256 31 / 25.5, 512 of L=512 88.8 / 81.1 (82.2 / 68.4), 96 of L=1300 93.2 / 92.5 (73.4 / 71.3),
+//                12 of L=5000 134 / 131 (99 / 76), 148 of L=2048 255 / 247 (172 / 159), 128 of L=4096 803 / 792
+//   grid:        8 of L=512 d=64 12.3 / 18.6, 40 of L=2048 101 / 122 (64.5 / 74.8), 20 of L=4000 167 / 212 (106 / 123),
+//                52 of L=1280 47 / 75 (43 / 57), 100 of L=700 46 / 54 (35 / 45), 60 of L=2700 198 / 227 (131 / 140),
+//                200 of L=768 75.5 / 81.6 (60.6 / 72.0)
+//   one each:    100 of L=1792 grid 140 / 156 (grid 102.1 / 106.2, where the rule picks the persistent one)
 struct FaFormCost {
   double grid, persistent;
 };
@@ -69,8 +70,8 @@ inline FaFormCost fa_form_cost(long long slices, int Lq, int Lkv, bool causal, i
 }
 
 // Long items (more than 40 KV blocks on average) take the grid form whatever the count: a static work list loses more to the
-// slowest SM than the boundaries cost. Without a mask / under a causal one, persistent against grid: L = 8192 0 % / +3 %,
-// B=16 H=32 L=16384 -2 % / -2 %, Lq=1024 x Lkv=16384 -3 %.
+// slowest SM than the boundaries cost. Grid / persistent, without a mask (causal): 16 slices of L=16384 1570 / 1887 (937 / 974),
+// 64 of L=8192 1535 / 1704, 32 of Lq=1024 Lkv=9000 122 / 252.
 inline bool fa_form_persistent(long long slices, int Lq, int Lkv, bool causal, int sms) {
   const int nblk = (Lkv + 127) / 128;
   if ((causal ? (nblk + 1) / 2 : nblk) > 40) return false;

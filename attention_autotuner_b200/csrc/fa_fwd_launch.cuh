@@ -27,8 +27,18 @@ struct FaFwdArgs {
   int causal;
 };
 
+// The default tile (two query tiles, up to 128 V columns, no softmax variant) is fa_fwd_persist_sm100.cuh's, in two forms of the
+// grid with the same bits.
 template <class Cfg>
-int fa_fwd_launch(const FaFwdArgs& a, cudaStream_t stream) {
+constexpr bool fa_fwd_default_tile() {
+  return Cfg::NQ == 2 && Cfg::SPLIT == 1 && Cfg::NMMA == 1 && Cfg::EXP_EMU == 0 && Cfg::EXP_H2 == 0 && Cfg::DV <= 128 && Cfg::NSTAGE >= 2;
+}
+template <class Cfg, bool SINGLE = false>
+int fa_fwd_persist_launch(const FaFwdArgs& a, cudaStream_t stream);
+
+// Every other tile: a grid of one CTA per 128 * NQ query rows.
+template <class Cfg>
+int fa_fwd_variant_launch(const FaFwdArgs& a, cudaStream_t stream) {
   if (!a.q || !a.k || !a.v || !a.o) return fail(kErrInvalidArgument, "fa_fwd: null tensor pointer");
   if (a.BH <= 0 || a.Lq <= 0 || a.Lkv <= 0) return fail(kErrInvalidArgument, "fa_fwd: sizes must be positive");
   if (a.BH > 65535) return fail(kErrInvalidArgument, "fa_fwd: batch*heads %d exceeds 65535", a.BH);
@@ -63,6 +73,13 @@ int fa_fwd_launch(const FaFwdArgs& a, cudaStream_t stream) {
   return check_launch("fa_fwd launch");
 }
 
+// The grid form of any tile.
+template <class Cfg>
+int fa_fwd_launch(const FaFwdArgs& a, cudaStream_t stream) {
+  if constexpr (fa_fwd_default_tile<Cfg>()) return fa_fwd_persist_launch<Cfg, true>(a, stream);
+  else return fa_fwd_variant_launch<Cfg>(a, stream);
+}
+
 // ATTN_B200_FA_FWD_FORM in the environment overrides the choice between the two forms of the kernel for every shape
 // they both cover: "grid" (one CTA per 256 query rows) or "persistent" (one CTA per SM walking a work list).
 inline int fa_fwd_form_requested() {  // 0: automatic, 1: grid, 2: persistent
@@ -80,8 +97,8 @@ inline int sm_count() {
   return sms;
 }
 
-// Launcher of the persistent kernel: one CTA per SM (fewer when there is less work) walking the work list.
-template <class Cfg>
+// Launcher of the default tile: one CTA per SM (fewer when there is less work) walking the work list, or one per work item.
+template <class Cfg, bool SINGLE>
 int fa_fwd_persist_launch(const FaFwdArgs& a, cudaStream_t stream) {
   if (!a.q || !a.k || !a.v || !a.o) return fail(kErrInvalidArgument, "fa_fwd: null tensor pointer");
   if (a.BH <= 0 || a.Lq <= 0 || a.Lkv <= 0) return fail(kErrInvalidArgument, "fa_fwd: sizes must be positive");
@@ -117,11 +134,11 @@ int fa_fwd_persist_launch(const FaFwdArgs& a, cudaStream_t stream) {
   if (n_super > 0x3fffffffLL) return fail(kErrInvalidArgument, "fa_fwd: too many tiles");
   pp.n_super = static_cast<int>(n_super);
 
-  auto kernel = &fa_fwd_persist_sm100_kernel<Cfg>;
+  auto kernel = &fa_fwd_persist_sm100_kernel<Cfg, SINGLE>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::SMEM_BYTES);
   if (e != cudaSuccess) return fail(kErrCuda, "fa_fwd: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   const int sms = sm_count();
-  const int grid = pp.n_super < sms ? pp.n_super : sms;
+  const int grid = SINGLE ? a.BH * pp.ndv * pp.nqb : pp.n_super < sms ? pp.n_super : sms;
   kernel<<<grid, Cfg::NTHREADS, Lay::SMEM_BYTES, stream>>>(tq, tk, tv, to, pp);
   return check_launch("fa_fwd launch");
 }
@@ -181,11 +198,10 @@ int fa_decode_launch(const FaFwdArgs& a, cudaStream_t stream) {
   return check_launch("fa_fwd launch");
 }
 
-// The default tile (two query tiles, up to 128 V columns, no softmax variant) exists in both forms, with the same bits; what
-// the persistent one saves lies at the boundaries of the work items. fa_fwd_form.cuh has the rule.
+// What the persistent form saves lies at the boundaries of the work items. fa_fwd_form.cuh has the rule.
 template <class Cfg>
 bool fa_fwd_picks_persistent(const FaFwdArgs& a) {
-  if constexpr (Cfg::NQ == 2 && Cfg::SPLIT == 1 && Cfg::NMMA == 1 && Cfg::EXP_EMU == 0 && Cfg::EXP_H2 == 0 && Cfg::DV <= 128) {
+  if constexpr (fa_fwd_default_tile<Cfg>()) {
     static_assert(Cfg::NQ * Cfg::BM == 256 && Cfg::BN == 128, "the rule's items and blocks");
     const int form = fa_fwd_form_requested();
     const long long slices = static_cast<long long>(a.BH) * (a.dv / Cfg::DV);
@@ -204,7 +220,7 @@ int fa_fwd_launch_auto(const FaFwdArgs& a, cudaStream_t stream) {
   if constexpr (Cfg::DQK == 64 || Cfg::DQK == 128) {
     if (fa_fwd_is_decode<Cfg>(a)) return fa_decode_launch<Cfg::DQK, Cfg::BF16>(a, stream);
   }
-  if constexpr (Cfg::NQ == 2 && Cfg::SPLIT == 1 && Cfg::NMMA == 1 && Cfg::EXP_EMU == 0 && Cfg::EXP_H2 == 0 && Cfg::DV <= 128) {
+  if constexpr (fa_fwd_default_tile<Cfg>()) {
     if (fa_fwd_picks_persistent<Cfg>(a)) return fa_fwd_persist_launch<Cfg>(a, stream);
   }
   return fa_fwd_launch<Cfg>(a, stream);

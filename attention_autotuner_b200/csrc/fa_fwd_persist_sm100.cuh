@@ -1,26 +1,47 @@
-// flash-attention forward for sm_100a, persistent form of fa_fwd_sm100_kernel (same tile, same roles, same
-// arithmetic): a grid of one CTA per SM walks a static work list instead of one CTA per 256 query rows.
+// flash-attention forward for sm_100a, the default tile: O = softmax(Q K^T * scale [+ causal mask]) V, LSE optional. Two
+// query tiles of 128 rows of one (batch, head) slice per work item, KV blocks of 128 keys, softmax as in fa_fwd_sm100.cuh (a
+// warpgroup per tile, thread t owns row t), the same arithmetic in the same order.
 //
-// What the non-persistent kernel pays per CTA -- launch, tensor-memory allocation, barrier set-up, the Q load, the
-// first S = Q K^T before any softmax can start, and at the end a last P V and an epilogue under which nothing else
-// runs -- is about 3.4 KV blocks' worth of time (measured through the causal case, whose CTAs average 16.5 blocks
-// at L = 4096 instead of 32, and through longer sequences). Here tensor memory and barriers live for the whole
-// kernel; the Q tiles of the next work item are loaded as soon as the last S MMA of the current one has read them;
-// the MMA warp goes straight from the last P V of one item to the first S of the next, so one query tile's epilogue
-// (tensor memory -> registers -> global) runs under the other tile's GEMMs and under its own next S.
+// What paces a tile is its chain S = Q K^T -> softmax -> O += P V -> next S. With P written over its S (fa_fwd_sm100.cuh)
+// the next S of a tile cannot start before its P V has read P, so a tile waits for both products (1024 tensor cycles and
+// the hand-offs between one issuing thread and two warpgroups, about 1480 cycles in an event trace) after every softmax
+// (2010 cycles), and the tensor pipe idles for 40 % of the time. Here P has columns of its own (tensor memory: S buffers,
+// P0, P1, O0, O1; at 128 columns of V that leaves ONE S buffer, which the tiles fill in turn): the threads of a tile load
+// their scores into registers and hand the buffer back at once (s_free), so that the next S runs under the softmax and
+// is there when the threads come for it. S and P V are issued by a warp each: a wait that is already over costs a thread
+// 80 cycles, a commit 65, a blocked issue hundreds, and in one thread that time adds up to more than the pipe's queue
+// covers (measured: this layout with one issuing warp 4500 cycles per block, 3490 before, 3000 with two).
+// Sustained / in a short burst, before and now, us (d = 128 fp16, bf16 where causal and not 4096): B=8 H=16 L=4096 1080 -> 944 /
+// 928 -> 815; causal 597 -> 544 / 516 -> 472; B=1 H=16 L=16384 causal 1123 -> 965 / 1000 -> 844; B=4 H=16 L=2999 causal
+// 188 -> 175 / 178 -> 160; B=2 H=16 Lq=1024 Lkv=9000 causal 155 -> 123; B=1 H=32 L=8192 d=64 805 -> 731. Work items of one
+// short block gain nothing (2000 slices of L=64: 56 / 56 at d=128, 47 -> 50 at d=64: more hand-offs per item). What bounds
+// it now: the power limit (the SM clock falls to 1.4 GHz under it) and the exponentials of both tiles beside the rest of
+// the softmax (2500 cycles per block for the pair, of which this form takes 3000).
 //
-// Work list: items are (slice, V-column chunk, block of 256 query rows). Pairs of items of equal total cost (k-th
-// heaviest and k-th lightest query block of a slice under a causal mask) are handed out round-robin, so every CTA
-// gets the same work up to one pair, and neighbouring CTAs work on the same slice (K and V shared in L2).
+// The work list has two forms. SINGLE: a grid of one CTA per work item, latest query block first. Otherwise one CTA per SM
+// walks a static list: what a CTA costs once -- launch, tensor-memory allocation, barrier set-up, the Q load, the first S
+// before any softmax can start, and at the end a last P V and an epilogue under which nothing else runs -- is paid once
+// per SM, the Q tiles of the next work item are loaded as soon as the last S MMA of the current one has read them, the
+// next item's first S goes ahead of the current one's last P V, and one query tile's epilogue runs under the other tile's
+// GEMMs and its own next S.
+//
+// Work list of the persistent form: items are (slice, V-column chunk, block of 256 query rows). Pairs of items of equal
+// total cost (k-th heaviest and k-th lightest query block of a slice under a causal mask) are handed out round-robin, so
+// every CTA gets the same work up to one pair, and neighbouring CTAs work on the same slice (K and V shared in L2).
 // Replaces the reference kernels flashattn_fwd_regfuse (csrc/kernels/attention/regfuse/regfuse.h:48-455) and
 // flashattn_fwd_smemfuse (csrc/kernels/attention/smemfuse/smemfuse.h:61-614), like fa_fwd_sm100.cuh.
+//
+// No wait can be circular: S(g) of the CTA's g-th block (a block of one tile) waits for the scores of the buffer's last
+// product to be read, which waits for that tile's previous block only, i.e. for P V before it; K of block r + 1 precedes V of
+// block r in the ring, and either is released by the product that reads it. K and V tiles report to barriers of their own
+// although they share the slots: a warp that waits for one kind only must not find the barrier a phase behind or ahead.
 #pragma once
 
 #include "fa_fwd_sm100.cuh"
 
 namespace ab200 {
 
-enum FaPersistTag : int { kTagQFree = 8, kTagOFree = 9 };
+enum FaPersistTag : int { kTagQFree = 8, kTagOFree = 9, kTagSFree = 10 };
 
 struct FaFwdPersistParams {
   FaFwdParams f;
@@ -35,23 +56,35 @@ struct FaFwdItem {
   int nmax;
 };
 
-// Output staging: where shared memory has room for both finished tiles (a K / V ring of up to three entries at
-// d = 128), a tile's rows are written there (16-bit, 128-byte swizzle) and leave through TMA stores, one per warp and
+// Output staging: where shared memory has room beside the operands (for both finished tiles with a K / V ring of up to three
+// entries at d = 128, for a box of each with four), a tile's rows are written there (16-bit, 128-byte swizzle) and leave through TMA stores, one per warp and
 // 64-column box (32 rows each, so no warp waits for another). A thread storing its own row writes 32-byte pieces of 32
 // different rows per instruction, which keeps the softmax warps from the next item's first block for as long as a
 // couple of KV blocks take.
 template <class Cfg>
 struct FaFwdPersistLayout {
-  static constexpr int O_TILE_BYTES = Cfg::BM * Cfg::DV * 2;
+  static constexpr int O_BOX_BYTES = Cfg::BM * 128;  // 128 rows x 64 columns
 #ifdef AB200_FA_FWD_NO_STAGE_O  // build option for comparisons: every thread stores its own row
-  static constexpr bool STAGE_O = false;
+  static constexpr int STAGE_BOXES = 0;
 #else
-  static constexpr bool STAGE_O = Cfg::DV % 64 == 0 && Cfg::SMEM_BYTES + 2 * O_TILE_BYTES <= 232448;
+  static constexpr int room(int boxes) { return Cfg::SMEM_BYTES + 64 + 2 * boxes * O_BOX_BYTES <= 232448; }
+  static constexpr int STAGE_BOXES = Cfg::DV % 64 != 0 ? 0 : room(Cfg::DV / 64) ? Cfg::DV / 64 : room(1) ? 1 : 0;
 #endif
-  static constexpr int SMEM_BYTES = Cfg::SMEM_BYTES + (STAGE_O ? 2 * O_TILE_BYTES : 0);
+  static constexpr bool STAGE_O = STAGE_BOXES > 0;
+  static constexpr int O_STAGE_BYTES = STAGE_BOXES * O_BOX_BYTES;  // per tile
+  static constexpr int MORE_BARRIERS = 64;  // beyond the 256 bytes of Cfg::SMEM_BYTES
+  static constexpr int SMEM_BYTES = Cfg::SMEM_BYTES + 2 * O_STAGE_BYTES + MORE_BARRIERS;
+  static_assert(SMEM_BYTES <= 232448, "shared memory overflow");
+  // Tensor memory (columns): score buffers, P of both tiles, O of both tiles.
+  static constexpr int S_BUFS = 2 * (128 + 64 + Cfg::DV) <= 512 ? 2 : 1;
+  static constexpr int P_COL = S_BUFS * 128;
+  static constexpr int O_COL = P_COL + 2 * 64;
+  static constexpr int COLS_USED = O_COL + 2 * Cfg::DV;
+  static constexpr int TMEM_COLS = COLS_USED <= 256 ? 256 : 512;
+  static_assert(COLS_USED <= 512, "tensor memory");
 };
 
-template <class Cfg>
+template <class Cfg, bool SINGLE>
 __global__ void __launch_bounds__(Cfg::NTHREADS, 1)
 fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                             const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -59,6 +92,7 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
   static_assert(Cfg::NQ == 2 && Cfg::SPLIT == 1 && Cfg::NMMA == 1 && Cfg::EXP_EMU == 0 && Cfg::EXP_H2 == 0,
                 "the persistent kernel is built for the default tile only");
   static_assert(Cfg::DV <= 128, "the epilogue holds a whole output row in registers");
+  static_assert(Cfg::NSTAGE >= 2, "K of the next block is loaded before V of the current one");
   constexpr int DQK = Cfg::DQK, DV = Cfg::DV, NQ = 2, NSTAGE = Cfg::NSTAGE;
   constexpr bool BF16 = Cfg::BF16;
   constexpr int BM = Cfg::BM, BN = Cfg::BN;
@@ -70,37 +104,47 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
   uint8_t* sKV = smem + NQ * Cfg::Q_TILE_BYTES;
   using Lay = FaFwdPersistLayout<Cfg>;
   constexpr bool STAGE_O = Lay::STAGE_O;
-  uint8_t* sO = smem + Cfg::SMEM_TILES;  // [2] finished tiles on their way out (STAGE_O only)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::SMEM_TILES + (STAGE_O ? 2 * Lay::O_TILE_BYTES : 0));
+  constexpr int S_BUFS = Lay::S_BUFS;
+  uint8_t* sO = smem + Cfg::SMEM_TILES;  // [2] finished tiles, or boxes of them, on their way out (STAGE_O only)
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::SMEM_TILES + 2 * Lay::O_STAGE_BYTES);
   uint64_t* q_full = bars;                   // [2] Q tile landed
   uint64_t* q_free = q_full + NQ;            // [2] the item's last S MMA of the tile is complete
-  uint64_t* kv_full = q_free + NQ;           // [NSTAGE]
-  uint64_t* kv_empty = kv_full + NSTAGE;     // [NSTAGE]
-  uint64_t* s_full = kv_empty + NSTAGE;      // [2]
-  uint64_t* p_full = s_full + NQ;            // [2]
+  uint64_t* k_full = q_free + NQ;            // [NSTAGE] a K tile landed in the slot
+  uint64_t* v_full = k_full + NSTAGE;        // [NSTAGE] a V tile did
+  uint64_t* kv_empty = v_full + NSTAGE;      // [NSTAGE]
+  uint64_t* s_full = kv_empty + NSTAGE;      // [2] per tile
+  uint64_t* s_free = s_full + NQ;            // [2] per score buffer: its scores are in registers
+  uint64_t* p_full = s_free + NQ;            // [2]
   uint64_t* o_done = p_full + NQ;            // [2]
   uint64_t* o_free = o_done + NQ;            // [2] the finished tile's O is in the softmax threads' registers
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(o_free + NQ);
   CtaAbort* ab = reinterpret_cast<CtaAbort*>(tmem_base_slot + 1);
-  static_assert((4 * NQ + 2 * NSTAGE + 4 * NQ) * 8 + 16 <= 256, "barrier area");
+  static_assert((7 * NQ + 3 * NSTAGE) * 8 + 16 <= 256 + Lay::MORE_BARRIERS, "barrier area");
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
-  constexpr int kMmaWarp = 4 * NQ;
-  constexpr int kTmaWarp = 4 * NQ + 1;
+  constexpr int kSWarp = 4 * NQ;
+  constexpr int kPvWarp = 4 * NQ + 1;
+  constexpr int kTmaWarp = 4 * NQ + 2;
 
   const int nblk_all = (p.Lkv + BN - 1) / BN;
   const int npair = (pp.nqb + 1) / 2;
-  const int n_steps = 2 * ((pp.n_super + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x));
+  const int n_steps = SINGLE ? 1 : 2 * ((pp.n_super + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x));
   // u-th work item of this CTA; false if there is none at this position
   auto get_item = [&](int u, FaFwdItem& it) -> bool {
-    const int sidx = (u >> 1) * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
-    if (sidx >= pp.n_super) return false;
-    const int j = sidx % npair;
     // heavy block first: under a causal mask the late query blocks see the most keys
-    const int qb = (u & 1) ? j : pp.nqb - 1 - j;
-    if ((u & 1) && qb == pp.nqb - 1 - j) return false;  // odd number of blocks: the middle one is alone
-    const int sl = sidx / npair;
+    int qb, sl;
+    if constexpr (SINGLE) {
+      sl = static_cast<int>(blockIdx.x) / pp.nqb;
+      qb = pp.nqb - 1 - static_cast<int>(blockIdx.x) % pp.nqb;
+    } else {
+      const int sidx = (u >> 1) * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
+      if (sidx >= pp.n_super) return false;
+      const int j = sidx % npair;
+      sl = sidx / npair;
+      qb = (u & 1) ? j : pp.nqb - 1 - j;
+      if ((u & 1) && qb == pp.nqb - 1 - j) return false;  // odd number of blocks: the middle one is alone
+    }
     it.bh = sl / pp.ndv;
     it.dv_off = (sl % pp.ndv) * DV;
     it.m_base = qb * (BM * NQ);
@@ -125,19 +169,21 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
       mbar_init(&q_full[i], 1);
       mbar_init(&q_free[i], 1);
       mbar_init(&s_full[i], 1);
-      mbar_init(&p_full[i], 128);
+      mbar_init(&s_free[i], 4);
+      mbar_init(&p_full[i], 4);
       mbar_init(&o_done[i], 1);
-      mbar_init(&o_free[i], 128);
+      mbar_init(&o_free[i], 4);
     }
     for (int i = 0; i < NSTAGE; ++i) {
-      mbar_init(&kv_full[i], 1);
+      mbar_init(&k_full[i], 1);
+      mbar_init(&v_full[i], 1);
       mbar_init(&kv_empty[i], 1);
     }
     ab->flag = 0;
     fence_mbar_init();
   }
-  if (warp == kMmaWarp) {
-    tmem_alloc(tmem_base_slot, Cfg::TMEM_COLS);
+  if (warp == kSWarp) {
+    tmem_alloc(tmem_base_slot, Lay::TMEM_COLS);
     tmem_relinquish();
   }
   if (warp == kTmaWarp && lane == 0) {
@@ -150,7 +196,7 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
 
-  if (warp >= kMmaWarp) {
+  if (warp >= kSWarp) {
     // 384 threads start with 168 registers each; the softmax threads take 208 (a 128-column score row), which
     // leaves this warpgroup 88: 256 x 208 + 128 x 88 = 384 x 168. (setmaxnreg.inc waits, with no limit, until the
     // registers it asks for have been released: the two numbers must add up to no more than the CTA was given.)
@@ -162,155 +208,189 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         bool ok = true;
         int t = 0;                 // ring items issued so far (all work items)
         int nq_loaded[NQ] = {0, 0};
-        for (int u = 0; u < n_steps && ok; ++u) {
+        uint32_t k_loads = 0, v_loads = 0;   // bit per slot: odd number of K / V tiles so far; 16 bits higher: any
+        // walks the (work item, block) pairs that have something to load
+        struct Walk {
+          int u, j;
           FaFwdItem it;
-          if (!get_item(u, it)) continue;
-          auto load_q = [&](int s) {
-            if (it.nblk[s] == 0 || !ok) return;
-            // the tile's buffer is free once the previous item's last S MMA of this tile has read it
-            if (nq_loaded[s] > 0) ok = mbar_wait(&q_free[s], (nq_loaded[s] - 1) & 1, ab, kTagQFree);
-            if (!ok) return;
-            mbar_expect_tx(&q_full[s], Cfg::Q_TILE_BYTES);
-#pragma unroll
-            for (int c = 0; c < DQK / 64; ++c)
-              tma_load_3d(sQ + s * Cfg::Q_TILE_BYTES + c * (BM * 128), &tmQ, &q_full[s], c * 64, it.m_base + s * BM, it.bh);
-            ++nq_loaded[s];
-          };
-          load_q(0);
-          // ring items of this work item: 2j = K block j, 2j+1 = V block j
-          for (int i = 0; i < 2 * it.nmax && ok; ++i, ++t) {
-            const int slot = t % NSTAGE;
-            const int use = t / NSTAGE;
-            if (use > 0) ok = mbar_wait(&kv_empty[slot], (use - 1) & 1, ab, kTagKvEmpty);
-            if (!ok) break;
-            uint8_t* dst = sKV + slot * Cfg::KV_SLOT_BYTES;
-            const int j = i >> 1;
-            if ((i & 1) == 0) {
-              mbar_expect_tx(&kv_full[slot], Cfg::K_TILE_BYTES);
-#pragma unroll
-              for (int c = 0; c < DQK / 64; ++c) tma_load_3d(dst + c * (BN * 128), &tmK, &kv_full[slot], c * 64, j * BN, it.bh);
-            } else {
-              mbar_expect_tx(&kv_full[slot], Cfg::V_TILE_BYTES);
-#pragma unroll
-              for (int c = 0; c < DV / 64; ++c)
-                tma_load_3d(dst + c * (BN * 128), &tmV, &kv_full[slot], it.dv_off + c * 64, j * BN, it.bh);
+        };
+        auto next_item = [&](Walk& w) -> bool {
+          while (++w.u < n_steps)
+            if (get_item(w.u, w.it) && w.it.nmax > 0) {
+              w.j = 0;
+              return true;
             }
-            if (i == 0) load_q(1);
+          return false;
+        };
+        auto load_q = [&](const FaFwdItem& it, int s) {
+          if (it.nblk[s] == 0 || !ok) return;
+          // the tile's buffer is free once the previous item's last S MMA of this tile has read it
+          if (nq_loaded[s] > 0) ok = mbar_wait(&q_free[s], (nq_loaded[s] - 1) & 1, ab, kTagQFree);
+          if (!ok) return;
+          mbar_expect_tx(&q_full[s], Cfg::Q_TILE_BYTES);
+#pragma unroll
+          for (int c = 0; c < DQK / 64; ++c)
+            tma_load_3d(sQ + s * Cfg::Q_TILE_BYTES + c * (BM * 128), &tmQ, &q_full[s], c * 64, it.m_base + s * BM, it.bh);
+          ++nq_loaded[s];
+        };
+        auto slot_free = [&]() -> uint8_t* {
+          const int slot = t % NSTAGE;
+          const int use = t / NSTAGE;
+          if (ok && use > 0) ok = mbar_wait(&kv_empty[slot], (use - 1) & 1, ab, kTagKvEmpty);
+          return sKV + slot * Cfg::KV_SLOT_BYTES;
+        };
+        auto load_k = [&](const Walk& w) {
+          uint8_t* dst = slot_free();
+          if (!ok) return;
+          uint64_t* bar = &k_full[t % NSTAGE];
+          k_loads = (k_loads ^ (1u << (t % NSTAGE))) | (0x10000u << (t % NSTAGE));
+          mbar_expect_tx(bar, Cfg::K_TILE_BYTES);
+#pragma unroll
+          for (int c = 0; c < DQK / 64; ++c) tma_load_3d(dst + c * (BN * 128), &tmK, bar, c * 64, w.j * BN, w.it.bh);
+          ++t;
+        };
+        auto load_v = [&](const Walk& w) {
+          uint8_t* dst = slot_free();
+          if (!ok) return;
+          uint64_t* bar = &v_full[t % NSTAGE];
+          v_loads = (v_loads ^ (1u << (t % NSTAGE))) | (0x10000u << (t % NSTAGE));
+          mbar_expect_tx(bar, Cfg::V_TILE_BYTES);
+#pragma unroll
+          for (int c = 0; c < DV / 64; ++c) tma_load_3d(dst + c * (BN * 128), &tmV, bar, w.it.dv_off + c * 64, w.j * BN, w.it.bh);
+          ++t;
+        };
+        Walk kw, vw;  // K runs one block ahead of V
+        kw.u = -1;
+        bool more = next_item(kw);
+        if (more) {
+          vw = kw;
+          load_q(kw.it, 0);
+          load_k(kw);
+          load_q(kw.it, 1);
+          while (ok) {
+            // K of the next block
+            bool new_item = false;
+            if (more && ++kw.j >= kw.it.nmax) {
+              more = next_item(kw);
+              new_item = more;
+            }
+            if (more) load_k(kw);
+            else ++t;  // V of block r is ring item 2 r + 2, also of the last one
+            // with two ring entries V's would wait for a block that the next item's Q tiles hold back
+            if (new_item && NSTAGE < 3)
+              for (int s = 0; s < NQ; ++s) load_q(kw.it, s);
+            // V of the current block
+            if (ok) load_v(vw);
+            if (new_item && NSTAGE >= 3)
+              for (int s = 0; s < NQ; ++s) load_q(kw.it, s);
+            if (++vw.j >= vw.it.nmax) {
+              if (!more) break;
+              vw = kw;
+            }
           }
         }
         if (!ok) {
           // abort path: let the copies already issued land before this CTA's shared memory is released
           for (int s = 0; s < NQ; ++s)
             if (nq_loaded[s] > 0) mbar_wait_drain(&q_full[s], (nq_loaded[s] - 1) & 1, 2000000ull);
-          for (int slot = 0; slot < NSTAGE; ++slot)
-            if (t > slot) mbar_wait_drain(&kv_full[slot], ((t - 1 - slot) / NSTAGE) & 1, 2000000ull);
+          for (int slot = 0; slot < NSTAGE; ++slot) {
+            if ((k_loads >> (16 + slot)) & 1u) mbar_wait_drain(&k_full[slot], ~(k_loads >> slot) & 1u, 2000000ull);
+            if ((v_loads >> (16 + slot)) & 1u) mbar_wait_drain(&v_full[slot], ~(v_loads >> slot) & 1u, 2000000ull);
+          }
         }
       }
-    } else if (warp == kMmaWarp) {
-      // ------------------------------------------------------------------ MMA issuer (converged warp, one elected lane)
+    } else if (warp == kSWarp) {
+      // ------------------------------------------------------------------ S = Q K^T (converged warp, one elected lane)
       constexpr uint32_t idesc_qk = umma_idesc(BM, BN, BF16, false, false);
-      constexpr uint32_t idesc_pv = umma_idesc(BM, DV, BF16, false, true);
+      const uint32_t q_desc = umma_desc_lo(smem_u32(sQ), 16), kv_desc = umma_desc_lo(smem_u32(sKV), 16);
       bool ok = true;
-      int t0 = 0;           // ring items of the work items before the current one
-      int full_waited = 0;  // ring items (global count) whose kv_full has been waited for
-      int n_items[NQ] = {0, 0};   // work items with at least one block, per tile, before the current one
-      int blk_done[NQ] = {0, 0};  // blocks of the tile in those items (phase base of p_full)
-      auto wait_item = [&](int t) -> bool {
-        while (ok && full_waited <= t) {
-          ok = mbar_wait_warp(&kv_full[full_waited % NSTAGE], (full_waited / NSTAGE) & 1, ab, kTagKvFull);
-          ++full_waited;
-        }
-        return ok;
-      };
-      const uint32_t q_addr = smem_u32(sQ);
-      const uint32_t kv_addr = smem_u32(sKV);
+      int slot = 0, r = 0;                  // ring slot of the block's K tile; blocks so far
+      uint32_t phases = 0;                  // bit per slot: phase of its next K tile
+      int n_s = 0;                          // products so far
+      int n_tile[NQ] = {0, 0};              // of either tile
+      int n_items[NQ] = {0, 0};             // work items with at least one block, per tile, before the current one
+      // (ring items: K of block r is number 2 r - 1, of the first one 0; V of block r number 2 r + 2)
       for (int u = 0; u < n_steps && ok; ++u) {
         FaFwdItem it;
         if (!get_item(u, it)) continue;
-        // S_s = Q_s K_j^T; releases the K slot if this tile is its last user, the Q tile after the tile's last block
-        auto issue_s = [&](int s, int j, bool release) {
-          const int slot = (t0 + 2 * j) % NSTAGE;
-          const uint32_t qa = q_addr + s * Cfg::Q_TILE_BYTES;
-          const uint32_t ka = kv_addr + slot * Cfg::KV_SLOT_BYTES;
-          const bool last_s = (j + 1 == it.nblk[s]);
-          if (elect_one()) {
+        for (int j = 0; j < it.nmax && ok; ++j) {
+          ok = mbar_wait_warp(&k_full[slot], (phases >> slot) & 1u, ab, kTagKvFull);
+          phases ^= 1u << slot;
+          const uint32_t kd = kv_desc + ((slot * Cfg::KV_SLOT_BYTES) >> 4);
+          const int last_user = it.nblk[1] > j ? 1 : 0;
 #pragma unroll
-            for (int ks = 0; ks < DQK / 16; ++ks) {
-              const uint32_t off = (ks >> 2) * (BM * 128) + (ks & 3) * 32;
-              umma_ss(tmem_base + s * 128, umma_smem_desc(qa + off, 16, 1024), umma_smem_desc(ka + off, 16, 1024),
-                      idesc_qk, ks > 0 ? 1u : 0u);
+          for (int s = 0; s < NQ; ++s) {
+            if (it.nblk[s] <= j || !ok) continue;
+            if (j == 0) ok = mbar_wait_warp(&q_full[s], n_items[s] & 1, ab, kTagQ);
+            // the buffer's scores are in the registers of the threads that read them last
+            const int before = S_BUFS == 1 ? n_s : n_tile[s];
+            if (ok && before > 0) ok = mbar_wait_warp(&s_free[S_BUFS == 1 ? 0 : s], (before - 1) & 1, ab, kTagSFree);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t qd = q_desc + ((s * Cfg::Q_TILE_BYTES) >> 4);
+            if (elect_one()) {
+#pragma unroll
+              for (int ks = 0; ks < DQK / 16; ++ks) {
+                const uint32_t off = ((ks >> 2) * (BM * 128) + (ks & 3) * 32) >> 4;
+                umma_ss(tmem_base + (S_BUFS == 1 ? 0 : s * 128), umma_desc(qd + off), umma_desc(kd + off), idesc_qk, ks > 0 ? 1u : 0u);
+              }
+              tc_commit(&s_full[s]);
+              if (s == last_user) tc_commit(&kv_empty[slot]);
+              if (j + 1 == it.nblk[s]) tc_commit(&q_free[s]);
             }
-            tc_commit(&s_full[s]);
-            if (release) tc_commit(&kv_empty[slot]);
-            if (last_s) tc_commit(&q_free[s]);
+            __syncwarp();
+            ++n_s;
+            ++n_tile[s];
           }
-          __syncwarp();
-        };
-        // O_s += P_s V_j; releases the V slot if this tile is its last user
-        auto issue_pv = [&](int s, int j, bool release) {
-          const int slot = (t0 + 2 * j + 1) % NSTAGE;
-          const uint32_t va = kv_addr + slot * Cfg::KV_SLOT_BYTES;
-          if (elect_one()) {
-#pragma unroll
-            for (int ks = 0; ks < BN / 16; ++ks)
-              umma_ts(tmem_base + NQ * 128 + s * DV, tmem_base + s * 128 + ks * 8,
-                      umma_smem_desc(va + ks * 2048, BN * 128, 1024), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
-            tc_commit(&o_done[s]);
-            if (release) tc_commit(&kv_empty[slot]);
-          }
-          __syncwarp();
-        };
-        int last_user = -1;
+          slot += r == 0 ? 1 : 2;
+          ++r;
+          if (slot >= NSTAGE) slot -= NSTAGE;
+        }
 #pragma unroll
         for (int s = 0; s < NQ; ++s)
-          if (it.nblk[s] > 0) last_user = s;
-        // prologue: S_s(0). The S columns of the tile are free: the last P V of the previous item has been issued.
-#pragma unroll
-        for (int s = 0; s < NQ; ++s) {
-          if (it.nblk[s] > 0 && ok) {
-            ok = mbar_wait_warp(&q_full[s], n_items[s] & 1, ab, kTagQ);
-            if (ok && wait_item(t0)) {
-              tc_fence_after();
-              issue_s(s, 0, s == last_user);
-            }
-          }
-        }
-        for (int j = 0; j < it.nmax && ok; ++j) {
-          // users of V_j are the tiles with nblk > j; users of K_{j+1} those with nblk > j+1
-          int last_v = -1, last_k = -1;
-#pragma unroll
-          for (int s = 0; s < NQ; ++s) {
-            if (it.nblk[s] > j) last_v = s;
-            if (it.nblk[s] > j + 1) last_k = s;
-          }
-#pragma unroll
-          for (int s = 0; s < NQ; ++s) {
-            if (it.nblk[s] > j && ok) {
-              if (!wait_item(t0 + 2 * j + 1)) break;
-              if (j == 0 && n_items[s] > 0) {
-                // the first P V of an item overwrites O: the previous item's epilogue must have read it
-                ok = mbar_wait_warp(&o_free[s], (n_items[s] - 1) & 1, ab, kTagOFree);
-                if (!ok) break;
-              }
-              // p_full of this tile completes once per block; blocks of earlier items are counted in its phase
-              ok = mbar_wait_warp(&p_full[s], (blk_done[s] + j) & 1, ab, kTagPFull);
-              if (!ok) break;
-              tc_fence_after();
-              issue_pv(s, j, s == last_v);
-            }
-            if (it.nblk[s] > j + 1 && ok) {
-              if (!wait_item(t0 + 2 * j + 2)) break;
-              tc_fence_after();
-              issue_s(s, j + 1, s == last_k);
-            }
-          }
-        }
-        t0 += 2 * it.nmax;
-#pragma unroll
-        for (int s = 0; s < NQ; ++s) {
           if (it.nblk[s] > 0) ++n_items[s];
-          blk_done[s] += it.nblk[s];
+      }
+    } else if (warp == kPvWarp) {
+      // ------------------------------------------------------------------ O += P V (converged warp, one elected lane)
+      constexpr uint32_t idesc_pv = umma_idesc(BM, DV, BF16, false, true);
+      const uint32_t kv_desc = umma_desc_lo(smem_u32(sKV), BN * 128);
+      bool ok = true;
+      int slot = 2 % NSTAGE;  // ring slot of the block's V tile
+      uint32_t phases = 0;    // bit per slot: phase of its next V tile
+      int n_tile[NQ] = {0, 0}, n_items[NQ] = {0, 0};
+      for (int u = 0; u < n_steps && ok; ++u) {
+        FaFwdItem it;
+        if (!get_item(u, it)) continue;
+        for (int j = 0; j < it.nmax && ok; ++j) {
+          ok = mbar_wait_warp(&v_full[slot], (phases >> slot) & 1u, ab, kTagKvFull);
+          phases ^= 1u << slot;
+          const uint32_t vd = kv_desc + ((slot * Cfg::KV_SLOT_BYTES) >> 4);
+          const int last_user = it.nblk[1] > j ? 1 : 0;
+#pragma unroll
+          for (int s = 0; s < NQ; ++s) {
+            if (it.nblk[s] <= j || !ok) continue;
+            // the first P V of an item overwrites O: the previous item's epilogue must have read it
+            if (j == 0 && n_items[s] > 0) ok = mbar_wait_warp(&o_free[s], (n_items[s] - 1) & 1, ab, kTagOFree);
+            if (ok) ok = mbar_wait_warp(&p_full[s], n_tile[s] & 1, ab, kTagPFull);
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) {
+#pragma unroll
+              for (int ks = 0; ks < BN / 16; ++ks)
+                umma_ts(tmem_base + Lay::O_COL + s * DV, tmem_base + Lay::P_COL + s * 64 + ks * 8, umma_desc(vd + ((ks * 2048) >> 4)),
+                        idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
+              tc_commit(&o_done[s]);
+              if (s == last_user) tc_commit(&kv_empty[slot]);
+            }
+            __syncwarp();
+            ++n_tile[s];
+          }
+          slot += 2;
+          if (slot >= NSTAGE) slot -= NSTAGE;
         }
+#pragma unroll
+        for (int s = 0; s < NQ; ++s)
+          if (it.nblk[s] > 0) ++n_items[s];
       }
     }
   } else {
@@ -319,8 +399,10 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
     const int s = warp >> 2;                    // query tile of this warpgroup
     const int row_in_tile = threadIdx.x & 127;  // TMEM lane
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32);
-    const uint32_t tS = tmem_addr(tmem_base, lane_base, s * 128);
-    const uint32_t tO = tmem_addr(tmem_base, lane_base, NQ * 128 + s * DV);
+    const uint32_t tS = tmem_addr(tmem_base, lane_base, S_BUFS == 1 ? 0 : s * 128);
+    const uint32_t tP = tmem_addr(tmem_base, lane_base, Lay::P_COL + s * 64);
+    const uint32_t tO = tmem_addr(tmem_base, lane_base, Lay::O_COL + s * DV);
+    uint64_t* my_s_free = &s_free[S_BUFS == 1 ? 0 : s];
     const int causal_shift = p.Lkv - p.Lq;
     bool ok = true;
     int cs = 0;  // blocks of this tile in the work items before the current one (phase base of s_full / o_done)
@@ -366,6 +448,10 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
           tmem_ld32(tS + 96, r + 96);
           tc_wait_ld();
         }
+        // the scores are in registers: the next product may overwrite their buffer
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(my_s_free);
         const int n0 = j * BN;
         // masking: keys past Lkv (ragged tail) and, under causal, keys j > i + shift
         const bool tail_blk = (n0 + BN > p.Lkv);
@@ -393,6 +479,11 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         mB = fmax3(mB, sv[BN - 2], sv[BN - 1]);
         const float m_blk = fmaxf(fmaxf(mA, mB), fmaxf(mC, mD));
 
+        // P V of this tile's previous block: O may be rescaled, and P overwritten, once it is complete
+        if (j > 0) {
+          ok = mbar_wait_warp(&o_done[s], (cs + j - 1) & 1, ab, kTagODone);
+          if (!ok) break;
+        }
         // Lazy rescale: keep the old reference unless the maximum grew by more than 2^8 in the exp2 domain.
         bool need = (j == 0) || ((m_blk - m_ref) * p.scale_log2 > Cfg::RESCALE_LOG2);
         if (m_blk == -INFINITY) need = false;
@@ -404,9 +495,6 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             l_sum *= alpha;
           }
           if (j > 0) {
-            // O of this tile was last written by PV(j-1): wait for it, then scale the rows in place.
-            ok = mbar_wait_warp(&o_done[s], (cs + j - 1) & 1, ab, kTagODone);
-            if (!ok) break;
             tc_fence_after();
 #pragma unroll
             for (int c0 = 0; c0 < DV; c0 += 32) {
@@ -436,7 +524,7 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             acc[(c >> 1) & 3] = fadd2(acc[(c >> 1) & 3], f2_pack(e0, e1));
             pk[c >> 1] = pack2<BF16>(e0, e1);
           }
-          tmem_st32(tS + h * (BN / 4), pk);
+          tmem_st32(tP + h * (BN / 4), pk);
         }
         {
           float a0, a1;
@@ -445,7 +533,8 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         }
         tc_wait_st();
         tc_fence_before();
-        mbar_arrive(&p_full[s]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[s]);
       }
       if (!ok) break;
       // epilogue: O / l -> global, lse. O goes to registers first so that the next item's first P V may overwrite it.
@@ -460,35 +549,39 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         for (int c0 = 0; c0 < DV; c0 += 32) tmem_ld32(tO + c0, r + c0);
         tc_wait_ld();
         tc_fence_before();
-        mbar_arrive(&o_free[s]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&o_free[s]);
         if constexpr (STAGE_O) {
           (void)orow;
-          // this warp's stores of the previous item must have read the staging rows before they are written again
-          if (lane == 0) tma_store_wait_read0();
-          __syncwarp();
-          uint8_t* stage = sO + s * Lay::O_TILE_BYTES + row_in_tile * 128;
 #pragma unroll
-          for (int i = 0; i < DV; i += 8) {
-            uint4 v;
-            v.x = pack2<BF16>(__uint_as_float(r[i + 0]) * inv_l, __uint_as_float(r[i + 1]) * inv_l);
-            v.y = pack2<BF16>(__uint_as_float(r[i + 2]) * inv_l, __uint_as_float(r[i + 3]) * inv_l);
-            v.z = pack2<BF16>(__uint_as_float(r[i + 4]) * inv_l, __uint_as_float(r[i + 5]) * inv_l);
-            v.w = pack2<BF16>(__uint_as_float(r[i + 6]) * inv_l, __uint_as_float(r[i + 7]) * inv_l);
-            const int chunk16 = (i & 63) >> 3;
-            *reinterpret_cast<uint4*>(stage + (i >> 6) * (BM * 128) + ((chunk16 ^ (row_in_tile & 7)) << 4)) = v;
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            FaFwdItem io;
-            get_item(u, io);
-            const int row0 = m_tile + (warp & 3) * 32;
-            if (row0 < p.Lq) {  // rows past the end of Q are clipped by the store
+          for (int b0 = 0; b0 < DV / 64; b0 += Lay::STAGE_BOXES) {
+            // this warp's earlier stores must have read the staging rows before they are written again
+            if (lane == 0) tma_store_wait_read0();
+            __syncwarp();
+            uint8_t* stage = sO + s * Lay::O_STAGE_BYTES + row_in_tile * 128;
 #pragma unroll
-              for (int b = 0; b < DV / 64; ++b)
-                tma_store_3d(&tmO, sO + s * Lay::O_TILE_BYTES + b * (BM * 128) + (warp & 3) * (32 * 128), io.dv_off + b * 64, row0,
-                             io.bh);
-              tma_store_commit();
+            for (int i = b0 * 64; i < (b0 + Lay::STAGE_BOXES) * 64; i += 8) {
+              uint4 v;
+              v.x = pack2<BF16>(__uint_as_float(r[i + 0]) * inv_l, __uint_as_float(r[i + 1]) * inv_l);
+              v.y = pack2<BF16>(__uint_as_float(r[i + 2]) * inv_l, __uint_as_float(r[i + 3]) * inv_l);
+              v.z = pack2<BF16>(__uint_as_float(r[i + 4]) * inv_l, __uint_as_float(r[i + 5]) * inv_l);
+              v.w = pack2<BF16>(__uint_as_float(r[i + 6]) * inv_l, __uint_as_float(r[i + 7]) * inv_l);
+              const int chunk16 = (i & 63) >> 3;
+              *reinterpret_cast<uint4*>(stage + ((i >> 6) - b0) * Lay::O_BOX_BYTES + ((chunk16 ^ (row_in_tile & 7)) << 4)) = v;
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              FaFwdItem io;
+              get_item(u, io);
+              const int row0 = m_tile + (warp & 3) * 32;
+              if (row0 < p.Lq) {  // rows past the end of Q are clipped by the store
+#pragma unroll
+                for (int b = 0; b < Lay::STAGE_BOXES; ++b)
+                  tma_store_3d(&tmO, sO + s * Lay::O_STAGE_BYTES + b * Lay::O_BOX_BYTES + (warp & 3) * (32 * 128),
+                               io.dv_off + (b0 + b) * 64, row0, io.bh);
+                tma_store_commit();
+              }
             }
           }
         } else if (row < p.Lq) {
@@ -513,9 +606,9 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
   __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (warp == kMmaWarp) {
+  if (warp == kSWarp) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+    tmem_dealloc(tmem_base, Lay::TMEM_COLS);
   }
 }
 

@@ -104,9 +104,7 @@ def kernel_of(workload):
         return "chain_pair_sm100_kernel"
     if workload in ATTN_BWD:
         return "fa_bwd_kv_sm100_kernel"
-    from attention_autotuner_b200.autotuner.cost_model import forward_is_persistent
-    B, H, Lq, Lkv, dqk, dv, dtype, causal = WORKLOADS[workload]
-    return "fa_fwd_persist_sm100_kernel" if forward_is_persistent(B * H, Lq, Lkv, causal) else "fa_fwd_sm100_kernel"
+    return "fa_fwd_persist_sm100_kernel"
 
 
 def flops_fwd(B, H, Lq, Lkv, dqk, dv, causal):
