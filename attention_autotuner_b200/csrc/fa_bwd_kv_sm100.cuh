@@ -223,13 +223,13 @@ fa_bwd_kv_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     }
     mbar_init(z1_full, 1);
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&w1_full[i], 256);
-      mbar_init(&w2_full[i], 256);
+      mbar_init(&w1_full[i], 8);
+      mbar_init(&w2_full[i], 8);
     }
     mbar_init(z2_full, 1);
     mbar_init(s_issued, 1);
     mbar_init(acc_done, 2);
-    mbar_init(acc_free, 128);
+    mbar_init(acc_free, 4);
     ab->flag = 0;
     fence_mbar_init();
   }
@@ -538,7 +538,7 @@ fa_bwd_kv_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
           tmem_st16(tz1 + h * 64, &pp[h * 16]);
           tc_wait_st();
           tc_fence_before();
-          mbar_arrive(&w1_full[h]);
+          mbar_arrive_warp(&w1_full[h]);
           if (threadIdx.x == 0) AB200_FBTR(0, g, 2 + h);
         }
         // ... then dS^T, both halves
@@ -556,7 +556,7 @@ fa_bwd_kv_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
           tmem_st16(tz2 + h * 64, pk);
           tc_wait_st();
           tc_fence_before();
-          mbar_arrive(&w2_full[h]);
+          mbar_arrive_warp(&w2_full[h]);
           if (threadIdx.x == 0) AB200_FBTR(0, g, 4 + h);
         }
         if (!ok) break;
@@ -592,7 +592,7 @@ fa_bwd_kv_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
           if (which == 1 && c0 + 32 >= D) {
             // both accumulators are in registers: the second GEMMs of the next work item may overwrite them
             tc_fence_before();
-            mbar_arrive(acc_free);
+            mbar_arrive_warp(acc_free);
           }
           if (grow < p.Lkv) {
 #pragma unroll

@@ -276,17 +276,17 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_const
     }
     for (int i = 0; i < 3; ++i) {
       mbar_init(&z_full[i], 1);
-      mbar_init(&w_full[i], 256);
+      mbar_init(&w_full[i], 8);
       mbar_init(&z_free[i], 1);
     }
     for (int i = 0; i < Cfg::NTAB; ++i) {
-      mbar_init(&tab_full[i], 128);
-      mbar_init(&tab_free[i], 256);
+      mbar_init(&tab_full[i], 4);
+      mbar_init(&tab_free[i], 8);
     }
     mbar_init(z2_full, 1);
-    mbar_init(z2_free, 256);
+    mbar_init(z2_free, 8);
     mbar_init(acc_done, 1);
-    mbar_init(acc_free, 128);
+    mbar_init(acc_free, 4);
     mbar_init(r_free, 1);
     ab->flag = 0;
     fence_mbar_init();
@@ -513,7 +513,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_const
             col_nl2[q] = tab[128 + (2 * grp + q) * 32 + lane];
             if (DUAL) col_nds[q] = tab[(2 * grp + q) * 32 + lane];
           }
-          mbar_arrive(&tab_free[ts]);
+          mbar_arrive_warp(&tab_free[ts]);
         }
         const bool diag = !SINGLES && p.causal && col0 == row0;  // the only block that straddles the diagonal (Lq == Lkv)
         if (threadIdx.x == 0) AB200_FBTR(0, g, 1);
@@ -582,7 +582,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_const
             if (q == 1) {
               // this thread's part of Z2 is in registers: the second GEMM1 of the next block may overwrite it
               tc_fence_before();
-              mbar_arrive(z2_free);
+              mbar_arrive_warp(z2_free);
               if (threadIdx.x == 0) AB200_FBTR(0, g, 5);
             }
             uint32_t pk[16];
@@ -614,7 +614,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_const
         }
         tc_wait_st();
         tc_fence_before();
-        mbar_arrive(&w_full[g % NZ]);
+        mbar_arrive_warp(&w_full[g % NZ]);
         if (threadIdx.x == 0) AB200_FBTR(0, g, 6);
       }
       if (!ok) break;
@@ -676,7 +676,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_const
         }
         tab[tid] = nds;
       }
-      mbar_arrive(&tab_full[ts]);
+      mbar_arrive_warp(&tab_full[ts]);
       if (tid == 0) AB200_FBTR(2, gp, 1);
       ++gp;
       if (++pt == pit.n_iter) p_next_item();
@@ -711,7 +711,7 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_const
         if (c0 + 32 >= D) {
           // the whole accumulator is in registers: GEMM2 of the next work item may overwrite it
           tc_fence_before();
-          mbar_arrive(acc_free);
+          mbar_arrive_warp(acc_free);
         }
         if (grow < rows_len) {
 #pragma unroll
