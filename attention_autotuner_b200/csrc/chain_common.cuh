@@ -66,9 +66,16 @@ __device__ __forceinline__ void chain_check_saturation(float abs_sum_so_far, con
 // Element-wise step of one block, W = Z .* mask .* scale (./ r), for the thread that owns TMEM lane (row) `tz >> 16`:
 // it reads fp32 values of its row of Z at `tz`, applies the row factor and the mask (decay factors built in
 // registers, or a general 16-bit mask tensor) and writes packed 16-bit pairs of W over the first columns of the same
-// buffer; the forward accumulates sum |W|. Every flavour handles two 32-column chunks (QD0, QD0 + 1) per call. With
-// SPLITW two threads share a row (chunks 0-1 and 2-3) and each keeps its 32 packed W columns inside its own half of
-// the buffer: W of chunks 0-1 at columns [0,32), of chunks 2-3 at [64,96); otherwise W sits at columns [0,64).
+// buffer; the forward accumulates sum |W|. Every flavour handles 64 columns from c0 on per call. With SPLITW two threads
+// share a row (columns from 0 and from 64) and each keeps its packed W columns inside its own half of the buffer: W of
+// columns 0-63 at [0,32), of 64-127 at [64,96); otherwise W sits at columns [0,64).
+//
+// c0 is a run-time value where two warpgroups work a block: they then run the same instructions, and an SM sub-partition,
+// which holds 32 KB of them (measured: straight-line code of one warp takes 1.0 cycles per instruction up to there and 2.6
+// beyond; two warps with 24 KB each 1.5 times as long as with the same 24 KB), keeps the step of both warpgroups beside an
+// MMA-issuing warp's. With a copy per warpgroup the step took 1000 (RowQ) to 2000 (Fwd) cycles per block in the kernels, twice
+// what it takes alone. B=8 H=8 L=2048 dqk=256 dv=512: forward 312 -> 296 us, backward 770 -> 730; with a mask tensor (B=4)
+// 201 -> 194 and 515 -> 510.
 //
 // Decay flavours (no mask tensor), written for instruction count and without shared-memory reads. Measured alone on
 // one SM, cycles per 128 x 128 block with two threads per row: 980 for a straightforward loop that reads a
@@ -81,23 +88,24 @@ __device__ __forceinline__ void chain_check_saturation(float abs_sum_so_far, con
 //     (colf0 / colf1 for the two chunks) and travels by warp shuffle;
 //   * both TMEM loads are issued before the first wait; the row sum uses four independent accumulators.
 // rowf is the per-row factor; lg = log2(gamma).
-template <int MODE, bool BF16, int QD0, bool SPLITW>
-__device__ __forceinline__ void chain_ew_decay2(uint32_t tz, float rowf, float lg, float colf0, float colf1, bool straddle,
+template <int MODE, bool BF16, bool SPLITW>
+__device__ __forceinline__ void chain_ew_decay2(uint32_t tz, int c0, float rowf, float lg, float colf0, float colf1, bool straddle,
                                                 int dlim, float& rsum) {
   uint32_t zr[2][32];
-  tmem_ld32(tz + QD0 * 32, zr[0]);
-  tmem_ld32(tz + (QD0 + 1) * 32, zr[1]);
+  tmem_ld32(tz + c0, zr[0]);
+  tmem_ld32(tz + c0 + 32, zr[1]);
   const uint64_t rf2 = f2_pack(rowf, rowf);
   const float ginv = exp2f(-lg);
   const uint64_t step2 = f2_pack(ginv * ginv, ginv * ginv);
   float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+  dlim -= c0;
   tc_wait_ld();
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
     uint32_t pk[16];
     uint64_t g = 0;
     if (MODE != kChainRowK) {
-      const float f0 = rowf * exp2f(-((QD0 + q) * 32) * lg);
+      const float f0 = rowf * exp2f(-(c0 + q * 32) * lg);
       g = f2_pack(f0, f0 * ginv);
     }
     const float colf = q == 0 ? colf0 : colf1;
@@ -120,7 +128,7 @@ __device__ __forceinline__ void chain_ew_decay2(uint32_t tz, float rowf, float l
       f2_unpack(a, w0, w1);
       f2_unpack(b, w2, w3);
       if (straddle) {  // warp-uniform: only blocks on the diagonal pay for the triangular predicate
-        const int cc = (QD0 + q) * 32 + 4 * c4;
+        const int cc = q * 32 + 4 * c4;
         if (MODE == kChainRowK) {
           if (cc < dlim) w0 = 0.f;
           if (cc + 1 < dlim) w1 = 0.f;
@@ -143,7 +151,7 @@ __device__ __forceinline__ void chain_ew_decay2(uint32_t tz, float rowf, float l
       pk[2 * c4 + 1] = pack2<BF16>(w2, w3);
     }
     if constexpr (MODE == kChainFwd && !BF16) chain_check_saturation((s0 + s1) + (s2 + s3), pk);
-    tmem_st16(tz + (SPLITW ? (QD0 >> 1) * 64 + q * 16 : (QD0 + q) * 16), pk);
+    tmem_st16(tz + (SPLITW ? c0 : c0 / 2) + q * 16, pk);
   }
   if (MODE == kChainFwd) rsum += (s0 + s1) + (s2 + s3);
 }
@@ -161,14 +169,14 @@ __device__ __forceinline__ float chain_rowk_colf(const ChainParams& p, int bh, i
 // The mask values a thread needs for one block are fetched BEFORE it waits for Z (their latency then runs under
 // GEMM1) and kept packed, two 16-bit values per register: mk[i] = columns (2i, 2i+1) of the thread's 64 columns.
 //   Fwd / RowQ: row `grow` of M[h], columns col0 + 32 QD0 ... : eight 16-byte loads.
-template <int MODE, int QD0>
+template <int MODE>
 __device__ __forceinline__ void chain_mask_prefetch(const ChainParams& p, int h, int grow, int col0, uint32_t (&mk)[32]) {
   static_assert(MODE != kChainRowK, "row reads only");
-  const uint16_t* mp = p.mask + (static_cast<size_t>(h) * p.Lq + grow) * p.Lkv + col0 + QD0 * 32;
+  const uint16_t* mp = p.mask + (static_cast<size_t>(h) * p.Lq + grow) * p.Lkv + col0;
 #pragma unroll
   for (int v8 = 0; v8 < 8; ++v8) {
     uint4 u = make_uint4(0, 0, 0, 0);
-    if (grow < p.Lq && col0 + QD0 * 32 + v8 * 8 < p.Lkv) u = __ldg(reinterpret_cast<const uint4*>(mp) + v8);
+    if (grow < p.Lq && col0 + v8 * 8 < p.Lkv) u = __ldg(reinterpret_cast<const uint4*>(mp) + v8);
     mk[4 * v8 + 0] = u.x;
     mk[4 * v8 + 1] = u.y;
     mk[4 * v8 + 2] = u.z;
@@ -178,13 +186,12 @@ __device__ __forceinline__ void chain_mask_prefetch(const ChainParams& p, int h,
 
 //   RowK with a transposed copy of the mask (mask_t[h][key][query], made once per backward call in scratch memory by
 //   mask_transpose_kernel): the thread's column of the mask is a row of the copy, read like the Fwd / RowQ rows.
-template <int QD0>
 __device__ __forceinline__ void chain_mask_prefetch_t(const ChainParams& p, int h, int key, int col0, uint32_t (&mk)[32]) {
-  const uint16_t* mp = p.mask_t + (static_cast<size_t>(h) * p.Lkv + key) * p.Lq + col0 + QD0 * 32;
+  const uint16_t* mp = p.mask_t + (static_cast<size_t>(h) * p.Lkv + key) * p.Lq + col0;
 #pragma unroll
   for (int v8 = 0; v8 < 8; ++v8) {
     uint4 u = make_uint4(0, 0, 0, 0);
-    if (key < p.Lkv && col0 + QD0 * 32 + v8 * 8 < p.Lq) u = __ldg(reinterpret_cast<const uint4*>(mp) + v8);
+    if (key < p.Lkv && col0 + v8 * 8 < p.Lq) u = __ldg(reinterpret_cast<const uint4*>(mp) + v8);
     mk[4 * v8 + 0] = u.x;
     mk[4 * v8 + 1] = u.y;
     mk[4 * v8 + 2] = u.z;
@@ -258,7 +265,6 @@ __global__ void __launch_bounds__(256) mask_transpose_kernel(const uint16_t* __r
 }
 
 // grow0 = first key of the warp (a multiple of 32); all 32 lanes of the warp must call this together.
-template <int QD0>
 __device__ __forceinline__ void chain_mask_prefetch_rowk(const ChainParams& p, int h, int grow0, int lane, int col0,
                                                          uint32_t (&mk)[32]) {
   const int kcol = grow0 + 8 * (lane >> 3);  // first of the 8 keys this lane reads
@@ -266,7 +272,7 @@ __device__ __forceinline__ void chain_mask_prefetch_rowk(const ChainParams& p, i
   for (int q = 0; q < 2; ++q) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int qi = col0 + (QD0 + q) * 32 + 8 * i + (lane & 7);
+      const int qi = col0 + q * 32 + 8 * i + (lane & 7);
       uint4 u = make_uint4(0, 0, 0, 0);
       if (qi < p.Lq && kcol < p.Lkv)
         u = __ldg(reinterpret_cast<const uint4*>(p.mask + (static_cast<size_t>(h) * p.Lq + qi) * p.Lkv + kcol));
@@ -292,12 +298,12 @@ __device__ __forceinline__ uint64_t chain_unpack_pair(uint32_t packed) {
 // for Z), no shared-memory reads; the forward accumulates sum |W|. RowK: times 1/r of the column, which travels by
 // shuffle from colf0 / colf1 (one column per lane and chunk) as in chain_ew_decay2.
 // Config 4 with a mask tensor: forward 0.31 against 0.35 ms with the loads issued after the wait.
-template <int MODE, bool BF16, int QD0, bool SPLITW>
-__device__ __forceinline__ void chain_ew_mask2(uint32_t tz, const uint32_t (&mk)[32], float rowf, float colf0, float colf1,
+template <int MODE, bool BF16, bool SPLITW>
+__device__ __forceinline__ void chain_ew_mask2(uint32_t tz, int c0, const uint32_t (&mk)[32], float rowf, float colf0, float colf1,
                                                float& rsum) {
   uint32_t zr[2][32];
-  tmem_ld32(tz + QD0 * 32, zr[0]);
-  tmem_ld32(tz + (QD0 + 1) * 32, zr[1]);
+  tmem_ld32(tz + c0, zr[0]);
+  tmem_ld32(tz + c0 + 32, zr[1]);
   const uint64_t rf2 = f2_pack(rowf, rowf);
   float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
   tc_wait_ld();
@@ -330,7 +336,7 @@ __device__ __forceinline__ void chain_ew_mask2(uint32_t tz, const uint32_t (&mk)
       pk[2 * c4 + 1] = pack2<BF16>(w2, w3);
     }
     if constexpr (MODE == kChainFwd && !BF16) chain_check_saturation((s0 + s1) + (s2 + s3), pk);
-    tmem_st16(tz + (SPLITW ? (QD0 >> 1) * 64 + q * 16 : (QD0 + q) * 16), pk);
+    tmem_st16(tz + (SPLITW ? c0 : c0 / 2) + q * 16, pk);
   }
   if (MODE == kChainFwd) rsum += (s0 + s1) + (s2 + s3);
 }

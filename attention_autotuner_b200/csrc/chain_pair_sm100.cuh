@@ -437,17 +437,13 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
         uint32_t mk[GENERAL ? 32 : 1];
         if constexpr (GENERAL && MODE != kChainRowK) {
           // the block's mask values of this thread (its row of the mask tensor), fetched before the wait for Z
-          if (hh == 0) chain_mask_prefetch<MODE, 0>(p, h, grow, col0, mk);
-          else chain_mask_prefetch<MODE, 2>(p, h, grow, col0, mk);
+          chain_mask_prefetch<MODE>(p, h, grow, col0 + hh * 64, mk);
         } else if constexpr (GENERAL) {
           // RowK: the thread's column of the mask, read by rows by the whole warp and transposed in registers
           if (p.mask_t != nullptr) {  // a transposed copy of the mask exists: the thread's column is a row of it
-            if (hh == 0) chain_mask_prefetch_t<0>(p, h, grow, col0, mk);
-            else chain_mask_prefetch_t<2>(p, h, grow, col0, mk);
-          } else if (hh == 0) {
-            chain_mask_prefetch_rowk<0>(p, h, grow - lane, lane, col0, mk);
+            chain_mask_prefetch_t(p, h, grow, col0 + hh * 64, mk);
           } else {
-            chain_mask_prefetch_rowk<2>(p, h, grow - lane, lane, col0, mk);
+            chain_mask_prefetch_rowk(p, h, grow - lane, lane, col0 + hh * 64, mk);
           }
         }
         float rowf = rowf_base;
@@ -463,11 +459,9 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
         tc_fence_after();
         const uint32_t tz = tmem_addr(tZ0 + (g & 1) * 128, lane_base, 0);
         if constexpr (GENERAL) {
-          if (hh == 0) chain_ew_mask2<MODE, BF16, 0, true>(tz, mk, rowf, colf0, colf1, rsum);
-          else chain_ew_mask2<MODE, BF16, 2, true>(tz, mk, rowf, colf0, colf1, rsum);
+          chain_ew_mask2<MODE, BF16, true>(tz, hh * 64, mk, rowf, colf0, colf1, rsum);
         } else {
-          if (hh == 0) chain_ew_decay2<MODE, BF16, 0, true>(tz, rowf, lg, colf0, colf1, straddle, dlim, rsum);
-          else chain_ew_decay2<MODE, BF16, 2, true>(tz, rowf, lg, colf0, colf1, straddle, dlim, rsum);
+          chain_ew_decay2<MODE, BF16, true>(tz, hh * 64, rowf, lg, colf0, colf1, straddle, dlim, rsum);
         }
         if (MODE == kChainFwd && t + 1 == n_iter) {
           // both halves add their partial row sums into the (zeroed) buffer the own epilogue reads; it must have

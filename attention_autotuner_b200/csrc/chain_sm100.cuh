@@ -431,15 +431,15 @@ chain_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constan
       // (Fwd / RowQ: its row of the mask; RowK: its column, read by rows by the whole warp and transposed)
       uint32_t mk0[GENERAL ? 32 : 1], mk1[GENERAL ? 32 : 1];
       if constexpr (GENERAL && MODE != kChainRowK) {
-        chain_mask_prefetch<MODE, 0>(p, h, grow, col0, mk0);
-        chain_mask_prefetch<MODE, 2>(p, h, grow, col0, mk1);
+        chain_mask_prefetch<MODE>(p, h, grow, col0, mk0);
+        chain_mask_prefetch<MODE>(p, h, grow, col0 + 64, mk1);
       } else if constexpr (GENERAL) {
         if (p.mask_t != nullptr) {  // a transposed copy of the mask exists: the thread's column is a row of it
-          chain_mask_prefetch_t<0>(p, h, grow, col0, mk0);
-          chain_mask_prefetch_t<2>(p, h, grow, col0, mk1);
+          chain_mask_prefetch_t(p, h, grow, col0, mk0);
+          chain_mask_prefetch_t(p, h, grow, col0 + 64, mk1);
         } else {
-          chain_mask_prefetch_rowk<0>(p, h, grow - lane, lane, col0, mk0);
-          chain_mask_prefetch_rowk<2>(p, h, grow - lane, lane, col0, mk1);
+          chain_mask_prefetch_rowk(p, h, grow - lane, lane, col0, mk0);
+          chain_mask_prefetch_rowk(p, h, grow - lane, lane, col0 + 64, mk1);
         }
       }
       float rowf = rowf_base;
@@ -456,11 +456,11 @@ chain_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constan
       tc_fence_after();
       const uint32_t tz = tmem_addr(tZ0 + (g & 1) * 128, lane_base, 0);
       if constexpr (GENERAL) {
-        chain_ew_mask2<MODE, BF16, 0, false>(tz, mk0, rowf, colf[0], colf[1], rsum);
-        chain_ew_mask2<MODE, BF16, 2, false>(tz, mk1, rowf, colf[2], colf[3], rsum);
+        chain_ew_mask2<MODE, BF16, false>(tz, 0, mk0, rowf, colf[0], colf[1], rsum);
+        chain_ew_mask2<MODE, BF16, false>(tz, 64, mk1, rowf, colf[2], colf[3], rsum);
       } else {
-        chain_ew_decay2<MODE, BF16, 0, false>(tz, rowf, lg, colf[0], colf[1], straddle, dlim, rsum);
-        chain_ew_decay2<MODE, BF16, 2, false>(tz, rowf, lg, colf[2], colf[3], straddle, dlim, rsum);
+        chain_ew_decay2<MODE, BF16, false>(tz, 0, rowf, lg, colf[0], colf[1], straddle, dlim, rsum);
+        chain_ew_decay2<MODE, BF16, false>(tz, 64, rowf, lg, colf[2], colf[3], straddle, dlim, rsum);
       }
       if (MODE == kChainFwd && t + 1 == n_iter) {
         // hand the row sums to the epilogue warpgroup (single buffer: the previous item's epilogue, which
