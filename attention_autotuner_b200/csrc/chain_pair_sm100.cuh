@@ -17,8 +17,12 @@
 //   7     scout: waits for this CTA's ring items and arrives on the LEADER's ready barriers (2 arrivals per group)
 //   8-11  element-wise warpgroup B: row t, columns [64,128)
 //   12-15 epilogue warpgroup: accumulator -> 16-bit -> shared memory -> TMA store
-// Two threads per row halve the latency of the element-wise step, which sits on the critical chain
-// GEMM1(t) -> W(t) -> GEMM2(t) -> GEMM1(t+2) (the block buffers in tensor memory are only two deep).
+// Tensor memory: Z (one buffer of 128 columns at N2 = 256, two at N2 = 128), W in two buffers of 64, ACC. The element-wise threads
+// load a block of Z into registers and hand the buffer back at once, so GEMM1 of the next block runs under their work and
+// under GEMM2; with W written over Z, in two buffers, GEMM1(t + 2) had to wait for GEMM2(t), and a chain of three hand-offs
+// (270 cycles to the MMA warps, 400 to 460 back) paced the kernel: 2750 (forward, dV) and 3750 (dK, dQ) cycles per block,
+// now 2150 and 3170 with 2048 and 3072 on the tensor pipe. B=8 H=8 L=2048 dqk=256 dv=512: forward 296 -> 280 us, backward 730
+// -> 693 (sustained; the SM clock falls to 1.5 GHz). What bounds it now: the power limit, and the boundaries of work items.
 // The epilogue stages its output in the ring slots that held the last T tile of the work item (GEMM2 leaves
 // them to the epilogue instead of returning them to the producer) and writes it with TMA stores: per-row
 // global stores from registers (one 32-byte sector per lane) kept the accumulator busy for ~4500 cycles and
@@ -56,11 +60,12 @@ struct ChainPairConfig {
   // (K1 = 512) in two rounds through the T slots only, so that the next item's first C tile is not held up.
   static constexpr bool ONE_ROUND = (CI >= TI) && (NSLOT >= 2 * (CI + TI));
   static constexpr int NTHREADS = 512;
-  static constexpr int TMEM_COLS = 512;  // 2 x 128 (Z) + N2
+  static constexpr int TMEM_COLS = 512;
+  static constexpr int Z_BUFS = N2 == 128 ? 2 : 1;  // Z_BUFS x 128 (Z) + 2 x 64 (W) + N2
   static_assert(K1 % 64 == 0 && K1 >= 64 && K1 <= 512, "K1");
   static_assert(N2 == 128 || N2 == 256, "N2");
   static_assert(NSLOT >= CI + TI, "ring too small");
-  static_assert(512 + (2 * NSLOT + 2 * NREADY + 14) * 8 + 16 <= AUX_BYTES, "barrier area");
+  static_assert(512 + (2 * NSLOT + 2 * NREADY + 16) * 8 + 16 <= AUX_BYTES, "barrier area");
 };
 
 template <class Cfg>
@@ -84,13 +89,14 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
   uint64_t* r_full = bars;                    // own    [1] resident tile landed (transaction count)
   uint64_t* slot_full = bars + 1;             // own    [NSLOT]
   uint64_t* slot_empty = slot_full + NSLOT;   // own    [NSLOT] slot may be refilled (commit from the leader, or the own epilogue)
-  uint64_t* z_full = slot_empty + NSLOT;      // own    [2] GEMM1 of a block complete
-  uint64_t* w_full = z_full + 2;              // leader [2] W written by the 512 element-wise threads of the pair
+  uint64_t* z_full = slot_empty + NSLOT;      // own    [2] GEMM1 of a block complete (per Z buffer)
+  uint64_t* w_full = z_full + 2;              // leader [2] W written by the 16 element-wise warps of the pair (per W buffer)
   uint64_t* acc_done = w_full + 2;            // own    [1] GEMM2 of a work item complete
   uint64_t* acc_free = acc_done + 1;          // leader [1] accumulators drained by the 256 epilogue threads
   uint64_t* r_free = acc_free + 1;            // own    [1] GEMM1 of a work item complete: R may be overwritten
-  uint64_t* z_free = r_free + 1;              // leader [2] GEMM2 of a block complete: its Z/W buffer may be rewritten
-  uint64_t* r_ready = z_free + 2;             // leader [1] resident tiles of both CTAs landed (2 arrivals)
+  uint64_t* z_free = r_free + 1;              // leader [2] Z is in the registers of the pair's 16 element-wise warps
+  uint64_t* w_free = z_free + 2;              // own    [2] GEMM2 of a block complete: its W buffer may be rewritten
+  uint64_t* r_ready = w_free + 2;             // leader [1] resident tiles of both CTAs landed (2 arrivals)
   uint64_t* rs_free = r_ready + 1;            // own    [1] forward: row sums consumed by the own epilogue (128 arrivals)
   uint64_t* c_ready = rs_free + 1;            // leader [NREADY] a C operand group landed in both CTAs (2 arrivals)
   uint64_t* t_ready = c_ready + NREADY;       // leader [NREADY] same for a T tile
@@ -142,8 +148,9 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&z_full[i], 1);
-      mbar_init(&w_full[i], 512);
-      mbar_init(&z_free[i], 1);
+      mbar_init(&w_full[i], 16);
+      mbar_init(&z_free[i], 16);
+      mbar_init(&w_free[i], 1);
     }
     mbar_init(acc_done, 1);
     mbar_init(acc_free, 256);
@@ -176,10 +183,14 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
   // The next kernel in the stream, if it was launched as a programmatic dependent (the backward's three kernels are
   // independent of each other), may take over SMs as this kernel's CTAs exit instead of waiting for the whole grid.
   pdl_launch_dependents();
-  const uint32_t tZ0 = tmem_base;          // Z buffers at columns [0,128) and [128,256); W overlays [0,32) and [64,96)
-  const uint32_t tACC = tmem_base + 256;   // [256, 256+N2)
+  // Tensor memory: ZB buffers of 128 columns for Z, two of 64 for W, the accumulators from column 256 (N2 = 256) or 384
+  constexpr int ZB = Cfg::Z_BUFS;
+  const uint32_t tZ0 = tmem_base;
+  const uint32_t tW0 = tmem_base + ZB * 128;
+  const uint32_t tACC = tW0 + 2 * 64;
   // leader's copies of the shared barriers, as shared::cluster addresses usable from both CTAs
   const uint32_t l_w_full = mapa_shared(smem_u32(w_full), 0);
+  const uint32_t l_z_free = mapa_shared(smem_u32(z_free), 0);
   const uint32_t l_acc_free = mapa_shared(smem_u32(acc_free), 0);
   const uint32_t l_c_ready = mapa_shared(smem_u32(c_ready), 0);
   const uint32_t l_t_ready = mapa_shared(smem_u32(t_ready), 0);
@@ -295,6 +306,7 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
     int cg = 0, tg = 0;  // operand groups consumed so far (as the scouts count them)
     const uint32_t r_addr = smem_u32(sR);
     const uint32_t ring_addr = smem_u32(sRing);
+    const uint32_t rd = umma_desc_lo(r_addr, 16);
     for (int u = 0; u < n_steps && ok; ++u) {
       ChainItem it;
       if (!decode_step(u, it)) continue;
@@ -305,13 +317,13 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
         if (lane == 0) AB200_CTR(1, kacc, 6);
         for (int t = 0; t < n && ok; ++t) {
           const int g = g0 + t;
-          if (g >= 2) {
-            // Z buffer g&1 still holds W(g-2) until GEMM2 of block g-2 has read it
-            ok = mbar_wait_warp(&z_free[g & 1], ((g - 2) >> 1) & 1, ab, kCtZFree);
+          if (g >= ZB) {
+            // the element-wise threads of both CTAs have the buffer's last block in registers
+            ok = mbar_wait_warp(&z_free[g % ZB], (g / ZB - 1) & 1, ab, kCtZFree);
             if (!ok) break;
           }
           if (lane == 0) AB200_CTR(1, g, 0);
-          const uint32_t tz = tZ0 + (g & 1) * 128;
+          const uint32_t tz = tZ0 + (g % ZB) * 128;
           const int base = b0 + (t == 0 ? 0 : CI + (t - 1) * (CI + TI));
 #pragma unroll
           for (int i0 = 0; i0 < CI; i0 += 2) {
@@ -324,15 +336,15 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
               for (int i = i0; i < i0 + 2; ++i) {
                 if (i < CI) {
                   const int slot = (base + i) % NSLOT;
-                  const uint32_t a = ring_addr + slot * ITEM;
+                  const uint32_t da = umma_desc_lo(ring_addr + slot * ITEM, 16);
                   const int nb = (K1B - 2 * i) >= 2 ? 2 : 1;
 #pragma unroll
                   for (int b = 0; b < 2; ++b) {
                     if (b < nb) {
 #pragma unroll
                       for (int ks = 0; ks < 4; ++ks)
-                        umma_ss2(tz, umma_smem_desc(r_addr + (2 * i + b) * TBOX + ks * 32, 16, 1024),
-                                 umma_smem_desc(a + b * CBOX + ks * 32, 16, 1024), idesc_z,
+                        umma_ss2(tz, umma_desc(rd + (((2 * i + b) * TBOX + ks * 32) >> 4)),
+                                 umma_desc(da + ((b * CBOX + ks * 32) >> 4)), idesc_z,
                                  (i > 0 || b > 0 || ks > 0) ? 1u : 0u);
                     }
                   }
@@ -341,7 +353,7 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
                 }
               }
               if (i0 + 2 >= CI) {
-                tc_commit2_both(&z_full[g & 1]);
+                tc_commit2_both(&z_full[g % ZB]);
                 if (t + 1 == n) tc_commit2_both(r_free);
               }
             }
@@ -363,7 +375,7 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
           ok = mbar_wait_warp(&w_full[g & 1], (g >> 1) & 1, ab, kCtWFull);
           if (!ok) break;
           if (lane == 0) AB200_CTR(1, g, 2);
-          const uint32_t tw = tZ0 + (g & 1) * 128;
+          const uint32_t tw = tW0 + (g & 1) * 64;
           const int base = b0 + CI + t * (CI + TI) + (t + 1 < n ? CI : 0);
           ok = mbar_wait_warp(&t_ready[tg % NREADY], (tg / NREADY) & 1, ab, kCtSlotFull);
           ++tg;
@@ -373,15 +385,15 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
 #pragma unroll
             for (int j = 0; j < TI; ++j) {
               const int slot = (base + j) % NSLOT;
-              const uint32_t a = ring_addr + slot * ITEM;
+              const uint32_t da = umma_desc_lo(ring_addr + slot * ITEM, TBOX);
 #pragma unroll
               for (int ks = 0; ks < 8; ++ks)
-                umma_ts2(tACC + j * 128, tw + (ks < 4 ? ks * 8 : 64 + (ks - 4) * 8), umma_smem_desc(a + ks * 2048, TBOX, 1024),
+                umma_ts2(tACC + j * 128, tw + ks * 8, umma_desc(da + ((ks * 2048) >> 4)),
                          idesc_acc, (t > 0 || ks > 0) ? 1u : 0u);
               // the slots of the last T tile go to the epilogues (output staging), which hand them back
               if (t + 1 < n) tc_commit2_both(&slot_empty[slot]);
             }
-            tc_commit2(smem_u32(&z_free[g & 1]));
+            tc_commit2_both(&w_free[g & 1]);
             if (t + 1 == n) tc_commit2_both(acc_done);
           }
           __syncwarp();
@@ -453,16 +465,27 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
         const int dlim = grow - col0;
 
         if (tid == 0 && hh == 0) AB200_CTR(0, g, 0);
-        ok = mbar_wait_warp(&z_full[g & 1], (g >> 1) & 1, ab, kCtZFull);
+        ok = mbar_wait_warp(&z_full[g % ZB], (g / ZB) & 1, ab, kCtZFull);
         if (!ok) break;
         if (tid == 0 && hh == 0) AB200_CTR(0, g, 1);
         tc_fence_after();
-        const uint32_t tz = tmem_addr(tZ0 + (g & 1) * 128, lane_base, 0);
+        const uint32_t tz = tmem_addr(tZ0 + (g % ZB) * 128, lane_base, 0);
+        const uint32_t tw = tmem_addr(tW0 + (g & 1) * 64, lane_base, hh * 32);
+        auto z_read = [&] {
+          tc_fence_before();
+          mbar_arrive_cluster_warp(l_z_free + (g % ZB) * 8);
+        };
+        auto w_ready = [&] {
+          if (g >= 2 && !mbar_wait_warp(&w_free[g & 1], ((g - 2) >> 1) & 1, ab, kCtWFree)) return false;
+          tc_fence_after();
+          return true;
+        };
         if constexpr (GENERAL) {
-          chain_ew_mask2<MODE, BF16, true>(tz, hh * 64, mk, rowf, colf0, colf1, rsum);
+          ok = chain_ew_mask2<MODE, BF16>(tz, tw, hh * 64, mk, rowf, colf0, colf1, rsum, z_read, w_ready);
         } else {
-          chain_ew_decay2<MODE, BF16, true>(tz, hh * 64, rowf, lg, colf0, colf1, straddle, dlim, rsum);
+          ok = chain_ew_decay2<MODE, BF16>(tz, tw, hh * 64, rowf, lg, colf0, colf1, straddle, dlim, rsum, z_read, w_ready);
         }
+        if (!ok) break;
         if (MODE == kChainFwd && t + 1 == n_iter) {
           // both halves add their partial row sums into the (zeroed) buffer the own epilogue reads; it must have
           // consumed the previous item's sums
@@ -475,7 +498,7 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
         if (tid == 0 && hh == 0) AB200_CTR(0, g, 2);
         tc_wait_st();
         tc_fence_before();
-        mbar_arrive_cluster(l_w_full + (g & 1) * 8);
+        mbar_arrive_cluster_warp(l_w_full + (g & 1) * 8);
         if (tid == 0 && hh == 0) AB200_CTR(0, g, 3);
       }
       if (!ok) break;

@@ -456,11 +456,11 @@ chain_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_constan
       tc_fence_after();
       const uint32_t tz = tmem_addr(tZ0 + (g & 1) * 128, lane_base, 0);
       if constexpr (GENERAL) {
-        chain_ew_mask2<MODE, BF16, false>(tz, 0, mk0, rowf, colf[0], colf[1], rsum);
-        chain_ew_mask2<MODE, BF16, false>(tz, 64, mk1, rowf, colf[2], colf[3], rsum);
+        chain_ew_mask2<MODE, BF16>(tz, tz, 0, mk0, rowf, colf[0], colf[1], rsum, [] {}, [] { return true; });
+        chain_ew_mask2<MODE, BF16>(tz, tz + 32, 64, mk1, rowf, colf[2], colf[3], rsum, [] {}, [] { return true; });
       } else {
-        chain_ew_decay2<MODE, BF16, false>(tz, 0, rowf, lg, colf[0], colf[1], straddle, dlim, rsum);
-        chain_ew_decay2<MODE, BF16, false>(tz, 64, rowf, lg, colf[2], colf[3], straddle, dlim, rsum);
+        chain_ew_decay2<MODE, BF16>(tz, tz, 0, rowf, lg, colf[0], colf[1], straddle, dlim, rsum, [] {}, [] { return true; });
+        chain_ew_decay2<MODE, BF16>(tz, tz + 32, 64, rowf, lg, colf[2], colf[3], straddle, dlim, rsum, [] {}, [] { return true; });
       }
       if (MODE == kChainFwd && t + 1 == n_iter) {
         // hand the row sums to the epilogue warpgroup (single buffer: the previous item's epilogue, which

@@ -39,6 +39,11 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t cta_addr, uint32_t rank
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// One arrival for a converged warp, as mbar_arrive_warp.
+__device__ __forceinline__ void mbar_arrive_cluster_warp(uint32_t cluster_addr) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive_cluster(cluster_addr);
+}
 
 // Tensor memory of the pair: the same columns are allocated in both CTAs. One warp of EACH CTA (the same
 // warp index) executes these.

@@ -420,8 +420,8 @@ ret_chunk_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       if (tid == 0) AB200_CTR(0, c, 0);
       {
         float unused_sum = 0.f;
-        chain_ew_decay2<kChainFwd, BF16, false>(tz, 0, row_decay, lg, 0.f, 0.f, true, tid, unused_sum);
-        chain_ew_decay2<kChainFwd, BF16, false>(tz, 64, row_decay, lg, 0.f, 0.f, true, tid, unused_sum);
+        chain_ew_decay2<kChainFwd, BF16>(tz, tz, 0, row_decay, lg, 0.f, 0.f, true, tid, unused_sum, [] {}, [] { return true; });
+        chain_ew_decay2<kChainFwd, BF16>(tz, tz + 32, 64, row_decay, lg, 0.f, 0.f, true, tid, unused_sum, [] {}, [] { return true; });
       }
       if (tid == 0) AB200_CTR(0, c, 1);
       // ---- the carried term Q S, now in ACC, seen from row i: times gamma^(i+1)
