@@ -325,14 +325,12 @@ fa_bwd_kv_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
     int g0 = 0, kacc = 0, n_held = 0;
     const uint32_t r1_addr = smem_u32(sR1), r2_addr = smem_u32(sR2), ring_addr = smem_u32(sRing), x_addr = smem_u32(sX);
     const uint32_t zero_addr = x_addr + (2 + NBX) * XB;
-    const uint64_t x1_desc = umma_smem_desc_noswizzle(x_addr, zero_addr - x_addr, 128);
-    const uint64_t x2_desc = umma_smem_desc_noswizzle(x_addr + XB, zero_addr - (x_addr + XB), 128);
-    // Descriptors are built once; an MMA's operand is its tile's descriptor plus a constant (the address field counts
-    // 16-byte units and no tile crosses the 256 KB the field can hold), so that issuing an MMA costs two additions.
-    const uint64_t d_r1 = umma_smem_desc(r1_addr, 16, 1024), d_r2 = umma_smem_desc(r2_addr, 16, 1024);
-    const uint64_t d_ring_k = umma_smem_desc(ring_addr, 16, 1024);    // streamed tile as K-major B operand (first GEMMs)
-    const uint64_t d_ring_mn = umma_smem_desc(ring_addr, BOX, 1024);  // streamed tile as MN-major B operand (second GEMMs)
-    const uint64_t d_bx = umma_smem_desc_noswizzle(x_addr + 2 * XB, zero_addr - (x_addr + 2 * XB), 128);  // term tile 0
+    const uint32_t d_x1 = umma_desc_lo(x_addr, zero_addr - x_addr), d_x2 = umma_desc_lo(x_addr + XB, zero_addr - (x_addr + XB));
+    // Low words of the descriptors, built once; an MMA's operand is its tile's plus a constant.
+    const uint32_t d_r1 = umma_desc_lo(r1_addr, 16), d_r2 = umma_desc_lo(r2_addr, 16);
+    const uint32_t d_ring_k = umma_desc_lo(ring_addr, 16);    // streamed tile as K-major B operand (first GEMMs)
+    const uint32_t d_ring_mn = umma_desc_lo(ring_addr, BOX);  // streamed tile as MN-major B operand (second GEMMs)
+    const uint32_t d_bx = umma_desc_lo(x_addr + 2 * XB, zero_addr - (x_addr + 2 * XB));  // term tile 0
     auto wait_item = [&](int item) {
       ok = mbar_wait_warp(&slot_full[item % NSLOT], (item / NSLOT) & 1, ab, kFkSlotFull);
     };
@@ -345,17 +343,17 @@ fa_bwd_kv_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
       if (!ok) return;
       if (lane == 0) AB200_FBTR(1, g, 2);
       const int slot = (2 * g) % NSLOT;
-      const uint64_t da = d_ring_k + ((slot * ITEM) >> 4);
+      const uint32_t da = d_ring_k + ((slot * ITEM) >> 4);
       // the term tile landed with the Q item of this block; a tile further on moves the zero tile one tile closer
-      const uint64_t dx = d_bx + (((g % NBX) * XB) >> 4) - (static_cast<uint64_t>(((g % NBX) * XB) >> 4) << 16);
+      const uint32_t dx = d_bx + (((g % NBX) * XB) >> 4) - ((static_cast<uint32_t>((g % NBX) * XB) >> 4) << 16);
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll MU
         for (int b = 0; b < DB; ++b)
 #pragma unroll MU
           for (int ks = 0; ks < 4; ++ks)
-            umma_ss(tZ1, d_r1 + ((b * BOX + ks * 32) >> 4), da + ((b * BOX + ks * 32) >> 4), idesc_z, (b > 0 || ks > 0) ? 1u : 0u);
-        umma_ss(tZ1, x1_desc, dx, idesc_z, 1u);
+            umma_ss(tZ1, umma_desc(d_r1 + ((b * BOX + ks * 32) >> 4)), umma_desc(da + ((b * BOX + ks * 32) >> 4)), idesc_z, (b > 0 || ks > 0) ? 1u : 0u);
+        umma_ss(tZ1, umma_desc(d_x1, kDescHiNoSwizzle), umma_desc(dx, kDescHiNoSwizzle), idesc_z, 1u);
         tc_commit(z1_full);
         tc_commit(&slot_empty[slot]);  // this warp's last use of the Q item (the other one: dK += W2 Q)
         if (last_of_item) tc_commit(r_free);
@@ -370,12 +368,12 @@ fa_bwd_kv_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
       if (!ok) return;
       if (lane == 0) AB200_FBTR(1, g, 4 + h);
       const int slot = (2 * g + 1) % NSLOT;
-      const uint64_t da = d_ring_mn + ((slot * ITEM + h * 4 * 2048) >> 4);
+      const uint32_t da = d_ring_mn + ((slot * ITEM + h * 4 * 2048) >> 4);
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll MU
         for (int j = 0; j < 4; ++j)
-          umma_ts(tACCV, tZ1 + w_col(h, j), da + ((j * 2048) >> 4), idesc_acc, (!first_of_item || h > 0 || j > 0) ? 1u : 0u);
+          umma_ts(tACCV, tZ1 + w_col(h, j), umma_desc(da + ((j * 2048) >> 4)), idesc_acc, (!first_of_item || h > 0 || j > 0) ? 1u : 0u);
         if (h == 1) {
           tc_commit(&slot_empty[slot]);  // this warp's last use of the dO item (the other one: Z2)
           if (last_of_item) tc_commit(acc_done);
@@ -389,16 +387,16 @@ fa_bwd_kv_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
       if (ok) wait_item(2 * g + 1);
       if (!ok) return;
       const int slot = (2 * g + 1) % NSLOT;
-      const uint64_t da = d_ring_k + ((slot * ITEM) >> 4);
-      const uint64_t dx = d_bx + (((g % NBX) * XB) >> 4) - (static_cast<uint64_t>(((g % NBX) * XB) >> 4) << 16);
+      const uint32_t da = d_ring_k + ((slot * ITEM) >> 4);
+      const uint32_t dx = d_bx + (((g % NBX) * XB) >> 4) - ((static_cast<uint32_t>((g % NBX) * XB) >> 4) << 16);
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll MU
         for (int b = 0; b < DB; ++b)
 #pragma unroll MU
           for (int ks = 0; ks < 4; ++ks)
-            umma_ss(tZ2, d_r2 + ((b * BOX + ks * 32) >> 4), da + ((b * BOX + ks * 32) >> 4), idesc_z, (b > 0 || ks > 0) ? 1u : 0u);
-        umma_ss(tZ2, x2_desc, dx, idesc_z, 1u);
+            umma_ss(tZ2, umma_desc(d_r2 + ((b * BOX + ks * 32) >> 4)), umma_desc(da + ((b * BOX + ks * 32) >> 4)), idesc_z, (b > 0 || ks > 0) ? 1u : 0u);
+        umma_ss(tZ2, umma_desc(d_x2, kDescHiNoSwizzle), umma_desc(dx, kDescHiNoSwizzle), idesc_z, 1u);
         tc_commit(z2_full);
         tc_commit(&slot_empty[slot]);
         if (last_of_item) tc_commit(r_free);
@@ -412,12 +410,12 @@ fa_bwd_kv_sm100_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_con
       if (!ok) return;
       if (lane == 0) AB200_FBTR(1, g, 6);
       const int slot = (2 * g) % NSLOT;  // full: Z2 of this block waited for it
-      const uint64_t da = d_ring_mn + ((slot * ITEM + h * 4 * 2048) >> 4);
+      const uint32_t da = d_ring_mn + ((slot * ITEM + h * 4 * 2048) >> 4);
       tc_fence_after();
       if (elect_one()) {
 #pragma unroll MU
         for (int j = 0; j < 4; ++j)
-          umma_ts(tACCK, tZ2 + w_col(h, j), da + ((j * 2048) >> 4), idesc_acc, (!first_of_item || h > 0 || j > 0) ? 1u : 0u);
+          umma_ts(tACCK, tZ2 + w_col(h, j), umma_desc(da + ((j * 2048) >> 4)), idesc_acc, (!first_of_item || h > 0 || j > 0) ? 1u : 0u);
         if (h == 1) {
           tc_commit(&slot_empty[slot]);
           if (last_of_item) tc_commit(acc_done);

@@ -363,7 +363,8 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_const
     constexpr uint32_t idesc_acc = umma_idesc(128, DB == 2 ? 128 : 64, BF16, false, true);
     bool ok = true;
     int b0 = 0, g0 = 0, kacc = 0;
-    const uint32_t r1_addr = smem_u32(sR1), r2_addr = smem_u32(sR2), ring_addr = smem_u32(sRing);
+    const uint32_t ring_addr = smem_u32(sRing);
+    const uint32_t d_r1 = umma_desc_lo(smem_u32(sR1), 16), d_r2 = umma_desc_lo(smem_u32(sR2), 16);
     for (int u = 0; u < n_steps && ok; ++u) {
       FaBwdItem it;
       if (!decode_step(u, it)) continue;
@@ -385,14 +386,14 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_const
             if (!ok) break;
             tc_fence_after();
             if (elect_one()) {
-              const uint32_t a = ring_addr + slot * ITEM;
+              const uint32_t da = umma_desc_lo(ring_addr + slot * ITEM, 16);
               const uint32_t tz = tZ1 + (g % NZ) * 128;
 #pragma unroll
               for (int b = 0; b < DB; ++b)
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks)
-                  umma_ss(tz, umma_smem_desc(r1_addr + b * BOX + ks * 32, 16, 1024),
-                          umma_smem_desc(a + b * BOX + ks * 32, 16, 1024), idesc_z, (b > 0 || ks > 0) ? 1u : 0u);
+                  umma_ss(tz, umma_desc(d_r1 + ((b * BOX + ks * 32) >> 4)),
+                          umma_desc(da + ((b * BOX + ks * 32) >> 4)), idesc_z, (b > 0 || ks > 0) ? 1u : 0u);
               tc_commit(&slot_empty[slot]);
               tc_commit(&z_full[g % NZ]);
               if (!DUAL && t + 1 == n) tc_commit(r_free);
@@ -412,13 +413,13 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_const
             if (!ok) break;
             tc_fence_after();
             if (elect_one()) {
-              const uint32_t a = ring_addr + slot * ITEM;
+              const uint32_t da = umma_desc_lo(ring_addr + slot * ITEM, 16);
 #pragma unroll
               for (int b = 0; b < DB; ++b)
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks)
-                  umma_ss(tZ2, umma_smem_desc(r2_addr + b * BOX + ks * 32, 16, 1024),
-                          umma_smem_desc(a + b * BOX + ks * 32, 16, 1024), idesc_z, (b > 0 || ks > 0) ? 1u : 0u);
+                  umma_ss(tZ2, umma_desc(d_r2 + ((b * BOX + ks * 32) >> 4)),
+                          umma_desc(da + ((b * BOX + ks * 32) >> 4)), idesc_z, (b > 0 || ks > 0) ? 1u : 0u);
               tc_commit(&slot_empty[slot]);
               tc_commit(z2_full);
               if (t + 1 == n) tc_commit(r_free);
@@ -443,11 +444,11 @@ fa_bwd_sm100_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_const
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
-            const uint32_t a = ring_addr + slot * ITEM;
+            const uint32_t da = umma_desc_lo(ring_addr + slot * ITEM, BOX);
             const uint32_t tw = tZ1 + (g % NZ) * 128;
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks)
-              umma_ts(tACC, tw + (ks < 4 ? ks * 8 : 64 + (ks - 4) * 8), umma_smem_desc(a + ks * 2048, BOX, 1024), idesc_acc, (t > 0 || ks > 0) ? 1u : 0u);
+              umma_ts(tACC, tw + (ks < 4 ? ks * 8 : 64 + (ks - 4) * 8), umma_desc(da + ((ks * 2048) >> 4)), idesc_acc, (t > 0 || ks > 0) ? 1u : 0u);
             tc_commit(&slot_empty[slot]);
             tc_commit(&z_free[g % NZ]);
             if (t + 1 == n) tc_commit(acc_done);

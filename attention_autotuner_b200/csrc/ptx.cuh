@@ -365,13 +365,14 @@ __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr, uint32_t lbo_
 
 // The same descriptor in two steps, for operands of one tile: the low word of the tile, to which an operand's offset is added in
 // units of 16 bytes (no tile crosses the 256 KB the address field can hold), and the constant high word.
-constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);  // rows of 128 bytes, 128-byte swizzle
+constexpr uint32_t kDescHiNoSwizzle = (128u >> 4) | (1u << 14);        // core matrices of 128 bytes one after another
 __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr, uint32_t lbo_bytes) {
   return ((saddr & 0x3FFFFu) >> 4) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);
 }
-__device__ __forceinline__ uint64_t umma_desc(uint32_t lo) {
+__device__ __forceinline__ uint64_t umma_desc(uint32_t lo, uint32_t hi = kDescHi) {
   uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(kDescHi));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
   return d;
 }
 
