@@ -24,6 +24,7 @@ struct ChainParams {
   int skip_upper;        // 1: blocks strictly above the diagonal are all zero and are skipped
   WorkList work;         // row blocks (128 rows; 256 for CTA pairs) of slices bh * ny + chunk
   int ny;                // column chunks of the output (n2_total / N2)
+  int wide;              // 1: rows of mask (Fwd, RowQ) or mask_t (RowK) start at multiples of 32 bytes
 };
 
 // One unit of work of the persistent chain kernel: a 128-row tile x one output-column chunk of one slice.
@@ -169,18 +170,32 @@ __device__ __forceinline__ float chain_rowk_colf(const ChainParams& p, int bh, i
   return f * exp2f(c * lg);
 }
 
-// ---- mask-tensor flavours, two 32-column chunks (QD0, QD0 + 1) per thread
+// ---- mask-tensor flavours, 64 columns per thread
 // The mask values a thread needs for one block are fetched BEFORE it waits for Z (their latency then runs under
 // GEMM1) and kept packed, two 16-bit values per register: mk[i] = columns (2i, 2i+1) of the thread's 64 columns.
-//   Fwd / RowQ: row `grow` of M[h], columns col0 + 32 QD0 ... : eight 16-byte loads.
-template <int MODE>
-__device__ __forceinline__ void chain_mask_prefetch(const ChainParams& p, int h, int grow, int col0, uint32_t (&mk)[32]) {
-  static_assert(MODE != kChainRowK, "row reads only");
-  const uint16_t* mp = p.mask + (static_cast<size_t>(h) * p.Lq + grow) * p.Lkv + col0;
+//   Fwd / RowQ: row `grow` of M[h], columns col0 ... col0 + 63.
+// Every lane reads a row of its own, so a load instruction touches 32 lines whatever its width, and two loads of 16 bytes fetch
+// the same 32-byte sector twice (eight warps' lines do not fit the L1 beside 227 KB of shared memory). Where the rows allow it
+// four loads of 32 bytes take the place of eight of 16 (B=4 H=8 L=2048 dqk=256 dv=512: forward 192 -> 184 us, backward 506 ->
+// 471).
+__device__ __forceinline__ void chain_mask_row(const uint16_t* mp, int valid, bool wide, uint32_t (&mk)[32]) {
+  if (wide) {
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      uint32_t* r = mk + 8 * v;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) r[i] = 0;
+      if (v * 16 < valid)
+        asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "l"(mp + v * 16));
+    }
+    return;
+  }
 #pragma unroll
   for (int v8 = 0; v8 < 8; ++v8) {
     uint4 u = make_uint4(0, 0, 0, 0);
-    if (grow < p.Lq && col0 + v8 * 8 < p.Lkv) u = __ldg(reinterpret_cast<const uint4*>(mp) + v8);
+    if (v8 * 8 < valid) u = __ldg(reinterpret_cast<const uint4*>(mp) + v8);
     mk[4 * v8 + 0] = u.x;
     mk[4 * v8 + 1] = u.y;
     mk[4 * v8 + 2] = u.z;
@@ -188,19 +203,16 @@ __device__ __forceinline__ void chain_mask_prefetch(const ChainParams& p, int h,
   }
 }
 
+template <int MODE>
+__device__ __forceinline__ void chain_mask_prefetch(const ChainParams& p, int h, int grow, int col0, uint32_t (&mk)[32]) {
+  static_assert(MODE != kChainRowK, "row reads only");
+  chain_mask_row(p.mask + (static_cast<size_t>(h) * p.Lq + grow) * p.Lkv + col0, grow < p.Lq ? p.Lkv - col0 : 0, p.wide != 0, mk);
+}
+
 //   RowK with a transposed copy of the mask (mask_t[h][key][query], made once per backward call in scratch memory by
 //   mask_transpose_kernel): the thread's column of the mask is a row of the copy, read like the Fwd / RowQ rows.
 __device__ __forceinline__ void chain_mask_prefetch_t(const ChainParams& p, int h, int key, int col0, uint32_t (&mk)[32]) {
-  const uint16_t* mp = p.mask_t + (static_cast<size_t>(h) * p.Lkv + key) * p.Lq + col0;
-#pragma unroll
-  for (int v8 = 0; v8 < 8; ++v8) {
-    uint4 u = make_uint4(0, 0, 0, 0);
-    if (key < p.Lkv && col0 + v8 * 8 < p.Lq) u = __ldg(reinterpret_cast<const uint4*>(mp) + v8);
-    mk[4 * v8 + 0] = u.x;
-    mk[4 * v8 + 1] = u.y;
-    mk[4 * v8 + 2] = u.z;
-    mk[4 * v8 + 3] = u.w;
-  }
+  chain_mask_row(p.mask_t + (static_cast<size_t>(h) * p.Lkv + key) * p.Lq + col0, key < p.Lkv ? p.Lq - col0 : 0, p.wide != 0, mk);
 }
 
 // RowK flavours: thread (lane L of its warp) owns key grow0 + L and needs M[h][query][key] for the 64 queries of its

@@ -167,6 +167,7 @@ inline ChainParams ret_params(const RetArgs& a) {
   p.Lkv = a.Lkv;
   p.scale = a.scale;
   p.skip_upper = (a.decay != nullptr || a.causal) ? 1 : 0;
+  p.wide = a.mask != nullptr && aligned32(a.mask) && a.Lkv % 16 == 0 ? 1 : 0;
   return p;
 }
 
@@ -228,12 +229,14 @@ int ret_bwd_launch(const RetArgs& a, cudaStream_t stream) {
     pv.out = a.dv_out;
     pv.ld_out = a.dv;
     pv.mask_t = mask_t;
+    pv.wide = mask_t != nullptr && aligned32(mask_t) && a.Lq % 16 == 0 ? 1 : 0;
     int r1 = chain_go<PAIR, DQK, DVC, kChainRowK, G, BF16>(a.k, a.Lkv, a.q, a.Lq, a.dout, a.dv, pv, a.BH, stream, "ret_bwd dV");
     if (r1) return r1;
     ChainParams pk = p;
     pk.out = a.dk;
     pk.ld_out = a.dqk;
     pk.mask_t = mask_t;
+    pk.wide = pv.wide;
     r1 = chain_go<PAIR, DV, DQC, kChainRowK, G, BF16>(a.v, a.Lkv, a.dout, a.Lq, a.q, a.dqk, pk, a.BH, stream, "ret_bwd dK", true);
     if (r1) return r1;
     ChainParams pq = p;

@@ -55,3 +55,24 @@ def test_sequences_of_blocks(form, dqk, dv, B, H, L):
     for b in range(0, B, max(1, B // 5)):
         one = run(*(t[b:b + 1].contiguous() for t in (q, k, v, do)), mask, decay)
         assert all(torch.equal(x[0], y[b]) for x, y in zip(one, got))
+
+
+@pytest.mark.parametrize("L,offset", [(128, 0), (136, 0), (144, 8), (272, 0)])
+def test_mask_rows_of_any_alignment(L, offset):
+    """Rows of the mask that start at multiples of 32 bytes are read by 32, others by 16: same values either way."""
+    B, H, dqk, dv = 2, 2, 128, 256
+    g = torch.Generator("cuda").manual_seed(3)
+    q, k, v, do = (torch.randn(B, H, L, d, generator=g, device="cuda").half() for d in (dqk, dqk, dv, dv))
+    store = torch.zeros(H * L * L + 16, device="cuda", dtype=torch.float16)
+    mask = store[offset:offset + H * L * L].view(H, L, L)  # offset 8: 16 bytes past a multiple of 32
+    mask.copy_(0.3 * torch.randn(H, L, L, generator=g, device="cuda"))
+    mask.tril_()
+    got = run(q, k, v, do, mask, None)
+    ref = mask.float().cpu()
+    args = [t.cpu() for t in (q, k, v)]
+    oref, rref = oracle.retnet_fwd(*args, ref, dqk ** -0.5)
+    assert oracle.within(oracle.error_stats(got[0].cpu(), oref), "fp16", scale_by_peak=True)
+    for mine, want in zip(got[2:], oracle.retnet_bwd(*args, ref, do.cpu(), dqk ** -0.5)):
+        assert oracle.within(oracle.error_stats(mine.cpu(), want), "fp16", scale_by_peak=True)
+    wide = mask.clone()  # the same values at the start of an allocation
+    assert all(torch.equal(x, y) for x, y in zip(got, run(q, k, v, do, wide, None)))
