@@ -36,7 +36,7 @@ constexpr bool fa_fwd_default_tile() {
 template <class Cfg, bool SINGLE = false>
 int fa_fwd_persist_launch(const FaFwdArgs& a, cudaStream_t stream);
 
-// Every other tile: a grid of one CTA per 128 * NQ query rows.
+// Every other tile, and work items of very few blocks: a grid of one CTA per 128 * NQ query rows.
 template <class Cfg>
 int fa_fwd_variant_launch(const FaFwdArgs& a, cudaStream_t stream) {
   if (!a.q || !a.k || !a.v || !a.o) return fail(kErrInvalidArgument, "fa_fwd: null tensor pointer");
@@ -73,11 +73,17 @@ int fa_fwd_variant_launch(const FaFwdArgs& a, cudaStream_t stream) {
   return check_launch("fa_fwd launch");
 }
 
-// The grid form of any tile.
+// The grid form of any tile. Items of one KV block (two where there is one query tile) have nothing to overlap and stay with
+// the kernel whose P lies over S: it has fewer hand-offs. That kernel / the other in us, d = 64 where not stated: 2 slices of
+// L=128 4.9 / 5.4, d=128 6.1 / 6.4, 100 of L=100 5.2 / 5.9, 4 of Lq=1000 Lkv=100 6.5 / 6.6, 1 of Lq=44 Lkv=255 6.4 / 6.7; with
+// more blocks 16 of Lq=1024 Lkv=256 7.8 / 7.8, Lkv=384 9.5 / 9.2, 4 of L=256 d=128 9.3 / 8.7, 8 of L=512 11.1 / 10.6. Same bits.
 template <class Cfg>
 int fa_fwd_launch(const FaFwdArgs& a, cudaStream_t stream) {
-  if constexpr (fa_fwd_default_tile<Cfg>()) return fa_fwd_persist_launch<Cfg, true>(a, stream);
-  else return fa_fwd_variant_launch<Cfg>(a, stream);
+  if constexpr (fa_fwd_default_tile<Cfg>()) {
+    const bool few_blocks = a.Lkv <= Cfg::BN || (a.Lq <= Cfg::BM && a.Lkv <= 2 * Cfg::BN);
+    if (!few_blocks) return fa_fwd_persist_launch<Cfg, true>(a, stream);
+  }
+  return fa_fwd_variant_launch<Cfg>(a, stream);
 }
 
 // ATTN_B200_FA_FWD_FORM in the environment overrides the choice between the two forms of the kernel for every shape
@@ -138,7 +144,7 @@ int fa_fwd_persist_launch(const FaFwdArgs& a, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::SMEM_BYTES);
   if (e != cudaSuccess) return fail(kErrCuda, "fa_fwd: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   const int sms = sm_count();
-  const int grid = SINGLE ? a.BH * pp.ndv * pp.nqb : pp.n_super < sms ? pp.n_super : sms;
+  const dim3 grid = SINGLE ? dim3(pp.nqb, pp.ndv, a.BH) : dim3(pp.n_super < sms ? pp.n_super : sms);
   kernel<<<grid, Cfg::NTHREADS, Lay::SMEM_BYTES, stream>>>(tq, tk, tv, to, pp);
   return check_launch("fa_fwd launch");
 }

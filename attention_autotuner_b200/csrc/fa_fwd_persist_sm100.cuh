@@ -133,20 +133,21 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
   // u-th work item of this CTA; false if there is none at this position
   auto get_item = [&](int u, FaFwdItem& it) -> bool {
     // heavy block first: under a causal mask the late query blocks see the most keys
-    int qb, sl;
+    int qb;
     if constexpr (SINGLE) {
-      sl = static_cast<int>(blockIdx.x) / pp.nqb;
-      qb = pp.nqb - 1 - static_cast<int>(blockIdx.x) % pp.nqb;
+      qb = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);
+      it.bh = static_cast<int>(blockIdx.z);
+      it.dv_off = static_cast<int>(blockIdx.y) * DV;
     } else {
       const int sidx = (u >> 1) * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
       if (sidx >= pp.n_super) return false;
       const int j = sidx % npair;
-      sl = sidx / npair;
+      const int sl = sidx / npair;
       qb = (u & 1) ? j : pp.nqb - 1 - j;
       if ((u & 1) && qb == pp.nqb - 1 - j) return false;  // odd number of blocks: the middle one is alone
+      it.bh = sl / pp.ndv;
+      it.dv_off = (sl % pp.ndv) * DV;
     }
-    it.bh = sl / pp.ndv;
-    it.dv_off = (sl % pp.ndv) * DV;
     it.m_base = qb * (BM * NQ);
     it.nmax = 0;
 #pragma unroll
@@ -164,22 +165,14 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
     return true;
   };
 
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < NQ; ++i) {
-      mbar_init(&q_full[i], 1);
-      mbar_init(&q_free[i], 1);
-      mbar_init(&s_full[i], 1);
-      mbar_init(&s_free[i], 4);
-      mbar_init(&p_full[i], 4);
-      mbar_init(&o_done[i], 1);
-      mbar_init(&o_free[i], 4);
-    }
-    for (int i = 0; i < NSTAGE; ++i) {
-      mbar_init(&k_full[i], 1);
-      mbar_init(&v_full[i], 1);
-      mbar_init(&kv_empty[i], 1);
-    }
-    ab->flag = 0;
+  // (a barrier per thread: one after another they cost a short call 0.2 us)
+  constexpr int kBars = 7 * NQ + 3 * NSTAGE;
+  static_assert(kBars <= 64, "set up by the first two warps");
+  if (threadIdx.x < kBars) {
+    uint64_t* bar = bars + threadIdx.x;
+    const bool by_warps = (bar >= s_free && bar < s_free + NQ) || (bar >= p_full && bar < p_full + NQ) || bar >= o_free;
+    mbar_init(bar, by_warps ? 4 : 1);
+    if (threadIdx.x == 0) ab->flag = 0;
     fence_mbar_init();
   }
   if (warp == kSWarp) {
@@ -483,6 +476,7 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         if (j > 0) {
           ok = mbar_wait_warp(&o_done[s], (cs + j - 1) & 1, ab, kTagODone);
           if (!ok) break;
+          tc_fence_after();
         }
         // Lazy rescale: keep the old reference unless the maximum grew by more than 2^8 in the exp2 domain.
         bool need = (j == 0) || ((m_blk - m_ref) * p.scale_log2 > Cfg::RESCALE_LOG2);
@@ -495,7 +489,6 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             l_sum *= alpha;
           }
           if (j > 0) {
-            tc_fence_after();
 #pragma unroll
             for (int c0 = 0; c0 < DV; c0 += 32) {
               uint32_t r[32];

@@ -37,7 +37,8 @@ def forward(q, k, v, causal):
 # one tile only, a second tile with a block more or none, items of one to three blocks, several items per SM, keys that
 # end inside a block, causal rows without a key
 SHAPES = [(300, 64, 64, False), (300, 128, 129, False), (300, 129, 128, True), (200, 256, 256, True), (160, 300, 290, True),
-          (150, 513, 513, True), (320, 17, 400, False), (150, 384, 100, True), (5, 2300, 2300, True), (3, 200, 2050, False)]
+          (150, 513, 513, True), (320, 17, 400, False), (150, 384, 100, True), (5, 2300, 2300, True), (3, 200, 2050, False),
+          (3, 128, 256, True), (3, 129, 256, False), (3, 128, 257, False)]
 
 
 @pytest.mark.parametrize("form", ["grid", "persistent"])
