@@ -56,7 +56,8 @@ class AttnConfig(BaseConfig):
         slot = max(128 * self.Kd * 2, 128 * self.dv_chunk * 2)
         if self.cta_pair:
             return q + 2 * self.kv_stages * (slot // 2) + 1024 + 512
-        return q + self.kv_stages * slot + 1024 + 256 + (self.q_tiles * 3072 if self.softmax_split == 2 else 0)
+        barriers = max(256, -(-((7 * self.q_tiles + 3 * self.kv_stages) * 8 + 16) // 64) * 64)
+        return q + self.kv_stages * slot + 1024 + barriers + (self.q_tiles * 3072 if self.softmax_split == 2 else 0)
 
     def tmem_columns(self) -> int:
         return self.q_tiles * (128 + self.dv_chunk)

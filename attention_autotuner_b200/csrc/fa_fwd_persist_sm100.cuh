@@ -67,13 +67,12 @@ struct FaFwdPersistLayout {
 #ifdef AB200_FA_FWD_NO_STAGE_O  // build option for comparisons: every thread stores its own row
   static constexpr int STAGE_BOXES = 0;
 #else
-  static constexpr int room(int boxes) { return Cfg::SMEM_BYTES + 64 + 2 * boxes * O_BOX_BYTES <= 232448; }
+  static constexpr int room(int boxes) { return Cfg::SMEM_BYTES + 2 * boxes * O_BOX_BYTES <= 232448; }
   static constexpr int STAGE_BOXES = Cfg::DV % 64 != 0 ? 0 : room(Cfg::DV / 64) ? Cfg::DV / 64 : room(1) ? 1 : 0;
 #endif
   static constexpr bool STAGE_O = STAGE_BOXES > 0;
   static constexpr int O_STAGE_BYTES = STAGE_BOXES * O_BOX_BYTES;  // per tile
-  static constexpr int MORE_BARRIERS = 64;  // beyond the 256 bytes of Cfg::SMEM_BYTES
-  static constexpr int SMEM_BYTES = Cfg::SMEM_BYTES + 2 * O_STAGE_BYTES + MORE_BARRIERS;
+  static constexpr int SMEM_BYTES = Cfg::SMEM_BYTES + 2 * O_STAGE_BYTES;
   static_assert(SMEM_BYTES <= 232448, "shared memory overflow");
   // Tensor memory (columns): score buffers, P of both tiles, O of both tiles.
   static constexpr int S_BUFS = 2 * (128 + 64 + Cfg::DV) <= 512 ? 2 : 1;
@@ -119,7 +118,9 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
   uint64_t* o_free = o_done + NQ;            // [2] the finished tile's O is in the softmax threads' registers
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(o_free + NQ);
   CtaAbort* ab = reinterpret_cast<CtaAbort*>(tmem_base_slot + 1);
-  static_assert((7 * NQ + 3 * NSTAGE) * 8 + 16 <= 256 + Lay::MORE_BARRIERS, "barrier area");
+  constexpr int kBars = 7 * NQ + 3 * NSTAGE;
+  static_assert(kBars * 8 + 16 <= Cfg::BARRIER_BYTES, "barrier area");
+  static_assert(NSTAGE <= 16, "the producer keeps two bits per ring entry in a word");
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int lane = threadIdx.x & 31;
@@ -166,7 +167,6 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
   };
 
   // (a barrier per thread: one after another they cost a short call 0.2 us)
-  constexpr int kBars = 7 * NQ + 3 * NSTAGE;
   static_assert(kBars <= 64, "set up by the first two warps");
   if (threadIdx.x < kBars) {
     uint64_t* bar = bars + threadIdx.x;

@@ -78,7 +78,11 @@ struct FaFwdConfig {
   static constexpr int TMEM_COLS = TMEM_COLS_USED <= 32 ? 32 : TMEM_COLS_USED <= 64 ? 64 : TMEM_COLS_USED <= 128 ? 128 : TMEM_COLS_USED <= 256 ? 256 : 512;
   static constexpr int SMEM_TILES = NQ * Q_TILE_BYTES + NSTAGE * KV_SLOT_BYTES;
   static constexpr int XCHG_BYTES = SPLIT == 2 ? NQ * 3 * 2 * 128 * 4 : 0;  // row max (double buffered) and row sum exchange
-  static constexpr int SMEM_BYTES = SMEM_TILES + 1024 /*alignment slack*/ + 256 /*barriers*/ + XCHG_BYTES;
+  // Barriers, tensor-memory address and abort flag of either kernel that takes this tile (fa_fwd_persist_sm100_kernel has the
+  // more: seven per query tile and three per ring entry); 256 bytes hold up to five ring entries, twelve fit at d = 64.
+  static constexpr int BARRIER_NEED = ((7 * NQ + 3 * NSTAGE) * 8 + 16 + 63) / 64 * 64;
+  static constexpr int BARRIER_BYTES = BARRIER_NEED > 256 ? BARRIER_NEED : 256;
+  static constexpr int SMEM_BYTES = SMEM_TILES + 1024 /*alignment slack*/ + BARRIER_BYTES + XCHG_BYTES;
   static_assert(DQK % 64 == 0 && DV % 64 == 0, "head dims must be multiples of 64");
   static_assert(TMEM_COLS_USED <= 512, "TMEM overflow: NQ*(128+DV) must be <= 512 columns");
   static_assert(DV <= 256, "one PV MMA covers at most N=256");
@@ -123,7 +127,8 @@ fa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* turn = o_done + NQ;              // [2] issue turns of the two MMA warps (NMMA == 2)
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(turn + 2);
   CtaAbort* ab = reinterpret_cast<CtaAbort*>(tmem_base_slot + 1);
-  float* xchg = reinterpret_cast<float*>(smem + Cfg::SMEM_TILES + 256);  // [NQ][3][2][128], SPLIT == 2 only
+  static_assert((4 * NQ + 2 * NSTAGE + 2) * 8 + 8 <= Cfg::BARRIER_BYTES, "barrier area");
+  float* xchg = reinterpret_cast<float*>(smem + Cfg::SMEM_TILES + Cfg::BARRIER_BYTES);  // [NQ][3][2][128], SPLIT == 2 only
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // provably warp-uniform
   const int lane = threadIdx.x & 31;
