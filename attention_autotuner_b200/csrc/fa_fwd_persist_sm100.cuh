@@ -200,6 +200,7 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
       if (lane == 0) {
         bool ok = true;
         int t = 0;                 // ring items issued so far (all work items)
+        int n_k = 0, n_v = 0;      // K and V tiles of them (event trace)
         int nq_loaded[NQ] = {0, 0};
         uint32_t k_loads = 0, v_loads = 0;   // bit per slot: odd number of K / V tiles so far; 16 bits higher: any
         // walks the (work item, block) pairs that have something to load
@@ -217,9 +218,11 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         };
         auto load_q = [&](const FaFwdItem& it, int s) {
           if (it.nblk[s] == 0 || !ok) return;
+          AB200_TR(3, n_k, 4 + 2 * s);
           // the tile's buffer is free once the previous item's last S MMA of this tile has read it
           if (nq_loaded[s] > 0) ok = mbar_wait(&q_free[s], (nq_loaded[s] - 1) & 1, ab, kTagQFree);
           if (!ok) return;
+          AB200_TR(3, n_k, 5 + 2 * s);
           mbar_expect_tx(&q_full[s], Cfg::Q_TILE_BYTES);
 #pragma unroll
           for (int c = 0; c < DQK / 64; ++c)
@@ -235,22 +238,26 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         auto load_k = [&](const Walk& w) {
           uint8_t* dst = slot_free();
           if (!ok) return;
+          AB200_TR(3, n_k, 1);
           uint64_t* bar = &k_full[t % NSTAGE];
           k_loads = (k_loads ^ (1u << (t % NSTAGE))) | (0x10000u << (t % NSTAGE));
           mbar_expect_tx(bar, Cfg::K_TILE_BYTES);
 #pragma unroll
           for (int c = 0; c < DQK / 64; ++c) tma_load_3d(dst + c * (BN * 128), &tmK, bar, c * 64, w.j * BN, w.it.bh);
           ++t;
+          ++n_k;
         };
         auto load_v = [&](const Walk& w) {
           uint8_t* dst = slot_free();
           if (!ok) return;
+          AB200_TR(3, n_v, 3);
           uint64_t* bar = &v_full[t % NSTAGE];
           v_loads = (v_loads ^ (1u << (t % NSTAGE))) | (0x10000u << (t % NSTAGE));
           mbar_expect_tx(bar, Cfg::V_TILE_BYTES);
 #pragma unroll
           for (int c = 0; c < DV / 64; ++c) tma_load_3d(dst + c * (BN * 128), &tmV, bar, w.it.dv_off + c * 64, w.j * BN, w.it.bh);
           ++t;
+          ++n_v;
         };
         Walk kw, vw;  // K runs one block ahead of V
         kw.u = -1;
@@ -309,17 +316,20 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         for (int j = 0; j < it.nmax && ok; ++j) {
           ok = mbar_wait_warp(&k_full[slot], (phases >> slot) & 1u, ab, kTagKvFull);
           phases ^= 1u << slot;
+          if (lane == 0) AB200_TR(2, r, 0);
           const uint32_t kd = kv_desc + ((slot * Cfg::KV_SLOT_BYTES) >> 4);
           const int last_user = it.nblk[1] > j ? 1 : 0;
 #pragma unroll
           for (int s = 0; s < NQ; ++s) {
             if (it.nblk[s] <= j || !ok) continue;
             if (j == 0) ok = mbar_wait_warp(&q_full[s], n_items[s] & 1, ab, kTagQ);
+            if (lane == 0) AB200_TR(2, r, 1 + 3 * s);
             // the buffer's scores are in the registers of the threads that read them last
             const int before = S_BUFS == 1 ? n_s : n_tile[s];
             if (ok && before > 0) ok = mbar_wait_warp(&s_free[S_BUFS == 1 ? 0 : s], (before - 1) & 1, ab, kTagSFree);
             if (!ok) break;
             tc_fence_after();
+            if (lane == 0) AB200_TR(2, r, 2 + 3 * s);
             const uint32_t qd = q_desc + ((s * Cfg::Q_TILE_BYTES) >> 4);
             if (elect_one()) {
 #pragma unroll
@@ -332,6 +342,7 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
               if (j + 1 == it.nblk[s]) tc_commit(&q_free[s]);
             }
             __syncwarp();
+            if (lane == 0) AB200_TR(2, r, 3 + 3 * s);
             ++n_s;
             ++n_tile[s];
           }
@@ -350,13 +361,14 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
       bool ok = true;
       int slot = 2 % NSTAGE;  // ring slot of the block's V tile
       uint32_t phases = 0;    // bit per slot: phase of its next V tile
-      int n_tile[NQ] = {0, 0}, n_items[NQ] = {0, 0};
+      int n_tile[NQ] = {0, 0}, n_items[NQ] = {0, 0}, r = 0;
       for (int u = 0; u < n_steps && ok; ++u) {
         FaFwdItem it;
         if (!get_item(u, it)) continue;
         for (int j = 0; j < it.nmax && ok; ++j) {
           ok = mbar_wait_warp(&v_full[slot], (phases >> slot) & 1u, ab, kTagKvFull);
           phases ^= 1u << slot;
+          if (lane == 0) AB200_TR(4, r, 0);
           const uint32_t vd = kv_desc + ((slot * Cfg::KV_SLOT_BYTES) >> 4);
           const int last_user = it.nblk[1] > j ? 1 : 0;
 #pragma unroll
@@ -367,6 +379,7 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             if (ok) ok = mbar_wait_warp(&p_full[s], n_tile[s] & 1, ab, kTagPFull);
             if (!ok) break;
             tc_fence_after();
+            if (lane == 0) AB200_TR(4, r, 1 + 2 * s);
             if (elect_one()) {
 #pragma unroll
               for (int ks = 0; ks < BN / 16; ++ks)
@@ -376,8 +389,10 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
               if (s == last_user) tc_commit(&kv_empty[slot]);
             }
             __syncwarp();
+            if (lane == 0) AB200_TR(4, r, 2 + 2 * s);
             ++n_tile[s];
           }
+          ++r;
           slot += 2;
           if (slot >= NSTAGE) slot -= NSTAGE;
         }
@@ -429,8 +444,10 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
       float m_ref = -INFINITY;  // reference maximum (raw score units) the exponentials are taken against
       float l_sum = 0.f;        // running sum of exp
       for (int j = 0; j < n_my; ++j) {
+        if (row_in_tile == 0) AB200_TR(s, cs + j, 0);
         ok = mbar_wait_warp(&s_full[s], (cs + j) & 1, ab, kTagSFull);
         if (!ok) break;
+        if (row_in_tile == 0) AB200_TR(s, cs + j, 1);
         tc_fence_after();
         float sv[BN];
         {
@@ -445,6 +462,7 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(my_s_free);
+        if (row_in_tile == 0) AB200_TR(s, cs + j, 2);
         const int n0 = j * BN;
         // masking: keys past Lkv (ragged tail) and, under causal, keys j > i + shift
         const bool tail_blk = (n0 + BN > p.Lkv);
@@ -478,6 +496,7 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
           if (!ok) break;
           tc_fence_after();
         }
+        if (row_in_tile == 0) AB200_TR(s, cs + j, 3);
         // Lazy rescale: keep the old reference unless the maximum grew by more than 2^8 in the exp2 domain.
         bool need = (j == 0) || ((m_blk - m_ref) * p.scale_log2 > Cfg::RESCALE_LOG2);
         if (m_blk == -INFINITY) need = false;
@@ -528,12 +547,14 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&p_full[s]);
+        if (row_in_tile == 0) AB200_TR(s, cs + j, 4);
       }
       if (!ok) break;
       // epilogue: O / l -> global, lse. O goes to registers first so that the next item's first P V may overwrite it.
       ok = mbar_wait_warp(&o_done[s], (cs + n_my - 1) & 1, ab, kTagODone);
       if (!ok) break;
       tc_fence_after();
+      if (row_in_tile == 0) AB200_TR(s, cs + n_my - 1, 5);
       const float inv_l = l_sum > 0.f ? 1.0f / l_sum : 0.f;
       {
         uint16_t* orow = out_row();
@@ -544,6 +565,7 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&o_free[s]);
+        if (row_in_tile == 0) AB200_TR(s, cs + n_my - 1, 6);
         if constexpr (STAGE_O) {
           (void)orow;
 #pragma unroll
@@ -590,6 +612,7 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
       }
       if (row < p.Lq)
         if (float* l = lse_row()) *l = (l_sum > 0.f) ? (m_ref * p.scale + __logf(l_sum)) : -INFINITY;
+      if (row_in_tile == 0) AB200_TR(s, cs + n_my - 1, 7);
       cs += n_my;
     }
     if (STAGE_O && lane == 0) tma_store_wait0();  // all output written before the CTA's shared memory is released
