@@ -139,6 +139,8 @@ int fa_fwd_persist_launch(const FaFwdArgs& a, cudaStream_t stream) {
   const long long n_super = static_cast<long long>(a.BH) * pp.ndv * ((pp.nqb + 1) / 2);
   if (n_super > 0x3fffffffLL) return fail(kErrInvalidArgument, "fa_fwd: too many tiles");
   pp.n_super = static_cast<int>(n_super);
+  pp.by_npair = make_fast_div((pp.nqb + 1) / 2);
+  pp.by_ndv = make_fast_div(pp.ndv);
 
   auto kernel = &fa_fwd_persist_sm100_kernel<Cfg, SINGLE>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay::SMEM_BYTES);
