@@ -308,6 +308,18 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             // the buffer's scores are in the registers of the threads that read them last
             const int before = S_BUFS == 1 ? n_s : n_tile[s];
             if (ok && before > 0) ok = mbar_wait_warp(&s_free[S_BUFS == 1 ? 0 : s], (before - 1) & 1, ab, kTagSFree);
+            // With a score buffer per tile nothing else holds the tiles apart, and once both softmaxes are in step each slows the
+            // other's exponentials (event trace: 2070 -> 2290 cycles). Tile 1 starts a long item when tile 0 has written its first
+            // P: 8 slices of L=4500 at d = 64 60 -> 58 us, persistent 20 of L=4000 206 -> 195. Short items lose that wait (100 of
+            // L=700 causal 30.5 -> 31.2); without a mask they gain 2 % in the grid form from following tile 0's reads instead (200
+            // of L=768 67.5 -> 64.5 us), but lose up to 5 % with one, and in the persistent form.
+            if (S_BUFS == 2 && s == 1 && it.nblk[0] > j && ok) {
+              if (it.nblk[0] >= 8) {
+                if (j == 0) ok = mbar_wait_warp(&p_full[0], (n_tile[0] - 1) & 1, ab, kTagPFull);
+              } else if (SINGLE && !p.causal) {
+                ok = mbar_wait_warp(&s_free[0], (n_tile[0] - 1) & 1, ab, kTagSFree);
+              }
+            }
             if (!ok) break;
             tc_fence_after();
             if (lane == 0) AB200_TR(2, r, 2 + 3 * s);
