@@ -212,7 +212,7 @@ int ret_bwd_launch(const RetArgs& a, cudaStream_t stream) {
   p.r_in = a.r;
   // Mask tensor: the dV and dK kernels own keys and need columns of M[h][query][key]. With scratch memory at hand the
   // mask is transposed once per call (one coalesced pass over H * Lq * Lkv values) and those kernels read rows of the
-  // copy with 16-byte loads; without it every warp reads 32 x 32 tiles by rows and transposes them in registers
+  // copy with loads of 32 or 16 bytes, as its alignment allows; without it every warp reads 32 x 32 tiles by rows and transposes them in registers
   // (three shuffle rounds per 8 x 8 block, on the element-wise warps' critical path).
   const size_t mask_bytes = static_cast<size_t>(a.H) * a.Lq * a.Lkv * 2u;
   const uint16_t* mask_t = nullptr;

@@ -106,7 +106,7 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
   uint64_t* z_full = slot_empty + NSLOT;      // own    [2] GEMM1 of a block complete (per Z buffer)
   uint64_t* w_full = z_full + 2;              // leader [2] W written by the 16 element-wise warps of the pair (per W buffer)
   uint64_t* acc_done = w_full + 2;            // own    [1] GEMM2 of a work item complete
-  uint64_t* acc_free = acc_done + 1;          // leader [1] accumulators drained by the 256 epilogue threads
+  uint64_t* acc_free = acc_done + 1;          // leader [1] accumulators drained by the 8 epilogue warps of the pair
   uint64_t* r_free = acc_free + 1;            // own    [1] GEMM1 of a work item complete: R may be overwritten
   uint64_t* z_free = r_free + 1;              // leader [2] Z is in the registers of the pair's 16 element-wise warps
   uint64_t* w_free = z_free + 2;              // own    [2] GEMM2 of a block complete: its W buffer may be rewritten
@@ -318,7 +318,7 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
     constexpr uint32_t idesc_acc = umma_idesc(256, 128, BF16, false, true);
     bool ok = true;
     int b0 = 0;    // ring items of earlier work items
-    int g0 = 0;    // 128-wide blocks of earlier work items (selects Z buffer and ready barrier)
+    int g0 = 0;    // 128-wide blocks of earlier work items (selects Z and W buffers and ready barrier)
     int kacc = 0;  // non-empty work items finished so far
     int cg = 0, tg = 0;  // operand groups consumed so far (as the scouts count them)
     const uint32_t r_addr = smem_u32(sR);
@@ -455,7 +455,7 @@ chain_pair_sm100_kernel(const __grid_constant__ CUtensorMap tmR, const __grid_co
       }
 
       for (int t = 0; t < n_iter; ++t) {
-        const int g = g0 + t;  // running block index: Z buffer g & 1
+        const int g = g0 + t;  // running block index: Z buffer g % ZB, W buffer g & 1
         const int col0 = (t_start + t) * 128;
         float colf0 = 0.f, colf1 = 0.f;
         if (MODE == kChainRowK) {

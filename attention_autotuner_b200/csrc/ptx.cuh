@@ -365,26 +365,17 @@ __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr, uint32_t lbo_
 
 // The same descriptor in two steps, for operands of one tile: the low word of the tile, to which an operand's offset is added in
 // units of 16 bytes (no tile crosses the 256 KB the address field can hold), and the constant high word.
+// Without swizzle, for small K-major operands written by threads or by a plain bulk copy: the tile is made of core matrices of
+// 8 rows x 16 bytes stored contiguously; the low word's LBO is then the distance of the two core matrices of a 16-element K
+// slice, the high word's SBO (128 bytes here) that of 8-row groups.
 constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);  // rows of 128 bytes, 128-byte swizzle
-constexpr uint32_t kDescHiNoSwizzle = (128u >> 4) | (1u << 14);        // core matrices of 128 bytes one after another
+constexpr uint32_t kDescHiNoSwizzle = (128u >> 4) | (1u << 14);
 __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr, uint32_t lbo_bytes) {
   return ((saddr & 0x3FFFFu) >> 4) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);
 }
 __device__ __forceinline__ uint64_t umma_desc(uint32_t lo, uint32_t hi = kDescHi) {
   uint64_t d;
   asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
-  return d;
-}
-
-// The same descriptor without swizzle, for small K-major operands written by threads or by a plain bulk copy: the
-// tile is made of core matrices of 8 rows x 16 bytes stored contiguously (128 bytes each);
-//   LBO = bytes between the two core matrices of a 16-element K slice, SBO = bytes between 8-row groups.
-__device__ __forceinline__ uint64_t umma_smem_desc_noswizzle(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16;
-  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFFu) << 32;
-  d |= 1ull << 46;
   return d;
 }
 
