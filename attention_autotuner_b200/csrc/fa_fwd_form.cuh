@@ -27,19 +27,20 @@ inline bool fa_decode_shape(int dqk, int dv, int Lq, int Lkv) {
 //     unless the deal moves by one position of the slice's list per round (sms and the list's length without a common
 //     factor), as it does with one item per slice: then its share of middle items.
 // Constants fitted to 292 measurements of both forms of an earlier kernel, whose products of a tile waited for one another (10 to
-// 2000 slices, Lq 64 to 4500, Lkv to 4096, d = 64 and 128, with and without a mask); over 116 measurements of the present one
-// (5 to 2000 slices, Lq 64 to 16384, Lkv to 16384) the form picked is 0.3 % slower than the faster one on average, 8 % at worst
-// (96 slices of Lq=512, Lkv=4096, d=128). Comparing the rounds of pairs with those of items instead, whatever the blocks of
-// an item, cost 4.6 % on average and up to 42 %: with one item per slice both forms hold the same items, and short items gain
-// most at their boundaries.
+// 2000 slices, Lq 64 to 4500, Lkv to 4096, d = 64 and 128, with and without a mask); over 138 measurements of the present one
+// (8 to 2000 slices, Lq 64 to 5000, Lkv to 5000) the form picked is 0.2 % slower than the faster one on average, 13 % at worst.
+// Comparing the rounds of pairs with those of items instead, whatever the blocks of an item, cost the earlier kernel 4.6 %
+// on average and up to 42 %: with one item per slice both forms hold the same items, and short items gain most at their
+// boundaries.
 // Measured grid / persistent in us, without a mask (causal); d = 128 where not stated:
-//   persistent:  2000 slices of L=64 84 / 56 (84 / 56), 1000 of L=256 68 / 53, d=64 57.7 / 40.8 (57.5 / 43.2),
-//                400 of L=256 31 / 25.5, 512 of L=512 88.8 / 81.1 (82.2 / 68.4), 96 of L=1300 93.2 / 92.5 (73.4 / 71.3),
-//                12 of L=5000 134 / 131 (99 / 76), 148 of L=2048 255 / 247 (172 / 159), 128 of L=4096 803 / 792
-//   grid:        8 of L=512 d=64 12.3 / 18.6, 40 of L=2048 101 / 122 (64.5 / 74.8), 20 of L=4000 167 / 212 (106 / 123),
-//                52 of L=1280 47 / 75 (43 / 57), 100 of L=700 46 / 54 (35 / 45), 60 of L=2700 198 / 227 (131 / 140),
-//                200 of L=768 75.5 / 81.6 (60.6 / 72.0)
-//   one each:    100 of L=1792 grid 140 / 156 (grid 102.1 / 106.2, where the rule picks the persistent one)
+//   persistent:  2000 slices of L=64 73.4 / 52.5 (73.9 / 52.5), 1000 of L=256 65.6 / 48.2, d=64 57.6 / 40.6 (55.9 / 40.5),
+//                400 of L=256 30.0 / 22.0, 512 of L=512 89.4 / 78.9 (78.5 / 65.5), 96 of L=1300 91.7 / 88.8 (70.3 / 65.6),
+//                12 of L=5000 131.6 / 128.5 (95.8 / 70.2), 148 of L=2048 264 / 250 (175 / 161), 128 of L=4096 894 / 827
+//   grid:        8 of L=512 d=64 12.3 / 18.6, 40 of L=2048 86.4 / 103.5 (57.9 / 67.7), 20 of L=4000 158 / 198 (97.5 / 111),
+//                52 of L=1280 42.4 / 68.4 (38.0 / 50.6), 100 of L=700 41.8 / 49.6 (31.4 / 41.8), 60 of L=2700 202 / 225
+//                (127 / 133), 200 of L=768 71.5 / 73.4 (57.1 / 65.0), 100 of L=1792 143.8 / 151.4
+//   misses:      96 of Lq=512 Lkv=4096 107.5 / 121.4 and 256 of L=1024 causal 100.6 / 105.3, where the rule takes the
+//                persistent form; d=64 96 of Lq=512 Lkv=4096 causal 99 / 95, where it takes the grid
 struct FaFormCost {
   double grid, persistent;
 };

@@ -548,7 +548,7 @@ fa_fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
       tc_fence_after();
       if (row_in_tile == 0) AB200_TR(s, cs + n_my - 1, 5);
       const float inv_l = l_sum > 0.f ? 1.0f / l_sum : 0.f;
-      FaFwdItem io;  // decoded again: only the tile's row and block count stay live across the block loop
+      FaFwdItem io;  // decoded again (persistent form): only the tile's row and block count stay live across the block loop
       get_item(u, io);
       {
         uint32_t r[DV];
