@@ -78,8 +78,8 @@ EXTRA_SHORT = ("C4", "C3", "C2causal", "C2bf16", "C2bf16causal", "C3mask", "C4ma
 SUSTAINED = ("C2", "C4")
 SEED = 20240229
 # dram__bytes_read.sum + dram__bytes_write.sum per step from the ncu captures summarised under profiles/
-# (one file per kernel and workload); None where no capture was taken
-NCU_TRAFFIC_BYTES = {"C2": 516.2e6, "C3": 383.6e6, "C4": 1725.3e6}
+# (counters_of_the_present_kernels.md); None where no capture was taken
+NCU_TRAFFIC_BYTES = {"C2": 517.8e6, "C3": 381.9e6, "C4": 1679.1e6}
 
 
 def metric_name(workload):
