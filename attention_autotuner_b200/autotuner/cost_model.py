@@ -12,8 +12,8 @@ budgets derived from the kernel structure (they are what bounds the kernels, see
   * tensor-pipe cycles executed per (128-row tile, 128-key block), including the recomputation a narrow output
     chunk forces (Q K^T once per chunk of V columns),
   * MUFU cycles of the softmax (one exponential per score, 16 per clock and SM), split by how the tile's softmax is
-    organised (one or two query tiles ping-ponging, one or two warpgroups per tile) because those decide how much of
-    it hides under the other tile's GEMMs,
+    organised (one or two query tiles ping-ponging, one or two warpgroups per tile, P over its scores or beside them)
+    because those decide how much of it hides under the other tile's GEMMs,
   * the share of exponentials moved to the FMA pipes or to packed fp16,
   * the fixed hand-off cost per block (commit -> barrier -> waiting warp), which a deeper ring or a CTA pair changes,
 each multiplied by the number of blocks the launch executes and divided by SM count x clock. The weights are a
@@ -86,7 +86,7 @@ def blocks(problem: dict) -> float:
 
 
 FEATURES = {
-    "attn": ["tensor", "mufu_1tile", "mufu_2tile", "mufu_2tile_split", "exp_emu", "exp_h2", "handoff_shallow",
+    "attn": ["tensor", "mufu_1tile", "mufu_2tile", "mufu_2tile_own_p", "mufu_2tile_split", "exp_emu", "exp_h2", "handoff_shallow",
              "handoff_deep", "pair", "mma2", "per_cta"],
     "ret": ["tensor", "handoff", "single_cta", "per_item"],
     "ret_bwd": ["tensor", "handoff", "single_cta", "per_item"],
@@ -108,11 +108,13 @@ def features(op: str, cfg: dict, problem: dict) -> np.ndarray:
         stages = cfg.get("kv_stages", 4)
         pair = 1.0 if cfg.get("cta_pair", 0) else 0.0
         tiles = problem["B"] * problem["H"] * np.ceil(problem["Lq"] / 128.0) * passes / SM_COUNT / 1e6
+        # the default tile has a kernel of its own, whose P does not lie over S (csrc/fa_fwd_launch.cuh: fa_fwd_default_tile)
+        default_tile = (q_tiles == 2 and chunk <= 128 and split == 1 and not cfg.get("exp_emu", 0) and not cfg.get("exp_h2", 0)
+                        and cfg.get("mma_warps", 1) == 1 and not cfg.get("cta_pair", 0) and stages >= 2)
         # the persistent form of the grid has no per-CTA prologue / epilogue to pay; left to the launcher (-1) it is
         # taken where it is estimated to be the faster one
         persistent = cfg.get("persistent", -1)
-        if persistent == -1 and q_tiles == 2 and chunk <= 128 and split == 1 and not cfg.get("exp_emu", 0) \
-                and not cfg.get("exp_h2", 0) and cfg.get("mma_warps", 1) == 1 and not cfg.get("cta_pair", 0):
+        if persistent == -1 and default_tile:
             persistent = int(forward_is_persistent(int(problem["B"] * problem["H"] * passes), int(problem["Lq"]), int(problem["Lkv"]),
                                                    bool(problem.get("causal", False))))
         if persistent == 1:
@@ -120,7 +122,8 @@ def features(op: str, cfg: dict, problem: dict) -> np.ndarray:
         return np.array([
             nb * t_tensor,
             nb * t_mufu * (q_tiles == 1),
-            nb * t_mufu * (q_tiles == 2 and split == 1),
+            nb * t_mufu * (q_tiles == 2 and split == 1 and not default_tile),
+            nb * t_mufu * default_tile,
             nb * t_mufu * (q_tiles == 2 and split == 2),
             nb * t_mufu * emu,
             nb * t_mufu * h2,
